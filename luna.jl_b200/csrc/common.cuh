@@ -13,6 +13,10 @@
 
 namespace luna {
 
+// The CTA's dynamic shared memory, one symbol for every kernel and device function (the transforms
+// take byte offsets into it).
+extern __shared__ __align__(256) char dsm[];
+
 template <typename R> struct alignas(2 * sizeof(R)) cpx { R x, y; };
 
 template <typename R> __host__ __device__ __forceinline__ cpx<R> mk(R a, R b) { cpx<R> c; c.x = a; c.y = b; return c; }
@@ -61,9 +65,13 @@ template <> struct Swz<float> {
 #define TW_NLO 64
 #define TW_NHI (TW_MMAX / TW_NLO)
 
+// fine: exp(-2*pi*i*a/4096), a < TWS_N, each rounded once (the FP64 shared-memory transforms).
+#define TWS_N 1024
+
 template <typename R> struct TwTab {
     const cpx<R>* lo;
     const cpx<R>* hi;
+    const cpx<R>* fine;
 };
 
 // exp(-2*pi*i*a/TW_MMAX), conjugated for inverse transforms

@@ -57,7 +57,7 @@ struct DWs {
 
 __host__ __device__ inline size_t dist_smem_bytes(int No, size_t csize, int R = DIST_R) {
     const size_t Mb = (size_t)(No / 2) / R;
-    return LUNA_SMALL_BYTES + 2 * align_up((Mb + 16) * csize, 256) + 4 * align_up(Mb * csize, 256);
+    return (csize == 16 ? SmallBytes<double>::v : SmallBytes<float>::v) + 2 * align_up((Mb + 16) * csize, 256) + 4 * align_up(Mb * csize, 256);
 }
 
 template <typename Rl, int R>
@@ -71,7 +71,7 @@ __device__ void plan_dws(const LunaInst& I, char* smem, DWs<Rl>& d, const TwTab<
     const size_t c = sizeof(cpx<Rl>);
     const size_t Mb = (size_t)(I.No / 2) / R;
     const size_t bs = align_up((Mb + 16) * c, 256), bm = align_up(Mb * c, 256);
-    size_t off = LUNA_SMALL_BYTES;
+    size_t off = SmallBytes<Rl>::v;
     d.stg = reinterpret_cast<cpx<Rl>*>(smem + off);
     off += bs;
     d.ef = reinterpret_cast<cpx<Rl>*>(smem + off);
@@ -90,14 +90,6 @@ __device__ __forceinline__ void dsync() { dcg::this_cluster().sync(); }
 template <typename T>
 __device__ __forceinline__ T* drem(T* p, int r) {
     return dcg::this_cluster().map_shared_rank(p, r);
-}
-
-// In-place Stockham transform (natural order in and out) of one buffer of length Mb, in
-// radix-8 passes (Mb/8 threads active): fewer barrier-separated passes matter more than
-// the idle threads for the short sub-transforms of a cluster.
-template <typename Rl, bool INV>
-__device__ __forceinline__ void sub_fft_any(cpx<Rl>* b, int Mb, const TwTab<Rl>& tw) {
-    sub_fft<Rl, INV, 8>(b, Mb, tw);
 }
 
 // exp(-+2 pi i a / 2^lg) from the twiddle table (a reduced modulo 2^lg)
@@ -159,7 +151,7 @@ __device__ __noinline__ void dist_c2r(DWs<Rl>& d, int Mc, int Nw, LoadF&& load) 
         }
     }
     __syncthreads();
-    sub_fft_any<Rl, true>(d.fb, Mbc, d.tw);
+    fft_sub1<Rl, true>(d.fb, Mbc, d.tw);
     if (p) {
         for (int n1 = tid; n1 < Mbc; n1 += T) {
             const int pos = Swz<Rl>::f(n1);
@@ -270,7 +262,7 @@ __device__ __noinline__ void dist_r2c(DWs<Rl>& d, int Mc, int Nw, StoreF&& store
     }
     __syncthreads();
     }
-    sub_fft_any<Rl, false>(d.fb, Mbc, d.tw);
+    fft_sub1<Rl, false>(d.fb, Mbc, d.tw);
     dsync();
     const int po = (R - p) % R;
     const cpx<Rl>* fo = drem(d.fb, po);
@@ -421,7 +413,7 @@ __device__ __noinline__ void dist_raman_fwd(const LunaResp& rr, DWs<Rl>& d, int 
     }
     __syncthreads();
     }
-    sub_fft2<Rl, false, 8>(d.rb0, d.rb1, Mb, d.tw);
+    fft_sub2<Rl, false>(d.rb0, d.rb1, Mb, d.tw);
     // pairs (f, Mr - f) with f = 2R k + p; Zk/Zm are entries of the complex transform
     const cpx<Rl>* H = reinterpret_cast<const cpx<Rl>*>(rr.H);
     auto pair = [&](int f, cpx<Rl>* bk, int ik, cpx<Rl>* bm, int im) {
@@ -459,7 +451,7 @@ __device__ __noinline__ void dist_raman_fwd(const LunaResp& rr, DWs<Rl>& d, int 
         for (int k = tid; k < Mb; k += T) pair(2 * R * k + c, d.rb0, k, d.rb1, Mb - 1 - k);
     }
     __syncthreads();
-    sub_fft2<Rl, true, 8>(d.rb0, d.rb1, Mb, d.tw);
+    fft_sub2<Rl, true>(d.rb0, d.rb1, Mb, d.tw);
     for (int n1 = tid; n1 < Mb; n1 += T) {
         const int pos = Swz<Rl>::f(n1);
         if (pa) d.rb0[pos] = d.rb0[pos] * tw_pow<Rl, true>(d.tw, (unsigned)(pa * n1), lgMr);
@@ -786,6 +778,112 @@ __device__ __noinline__ void dist_plasma(const LunaInst& I, DWs<Rl>& d, int M, d
     __syncthreads();
 }
 
+// The FP64 form: NS consecutive samples of this CTA's block per thread, every quantity FP64, the
+// exchange of carries and first samples as in dist_plasma. The samples' rates, fractions and
+// currents stay in registers up to eight a thread (dist_plasma's passes over shared memory took
+// 1.2-1.8 kB of spill traffic in FP64) and the rates are evaluated together (rates_f64); a warp
+// without ionisation takes one exp for its samples and no loss current.
+template <int NS, int R>
+__device__ __noinline__ void dist_plasma_f64(const LunaInst& I, DWs<double>& d, int M, double sc, int ip, int ir,
+                                             double kc, double rc) {
+    const int q = d.rank, tid = threadIdx.x;
+    const int Mb = M / R, mbase = q * Mb;
+    const LunaResp& r = I.resp[ip];
+    const double dt = r.dt, er = r.eratio, coef = r.coef, ipot = r.ionpot, pre1 = r.preion + 1.0;
+    constexpr int G = NS < 8 ? NS : 8;  // samples evaluated together
+    const int pr0 = tid * (NS / 2);
+    double E[NS], rr[NS];
+#pragma unroll
+    for (int h = 0; h < NS / 2; ++h) {
+        const cpx<double> e = d.tb[Swz<double>::f(pr0 + h)];
+        E[2 * h] = e.x * sc;
+        E[2 * h + 1] = e.y * sc;
+    }
+    double acc = 0, tot;
+    bool ion = false;
+#pragma unroll
+    for (int g = 0; g < NS; g += G) {
+        rates_f64<G>(r, E + g, d.flag, rr + g);
+#pragma unroll
+        for (int s = 0; s < G; ++s) {
+            acc += rr[g + s];
+            ion = ion || rr[g + s] != 0.0;
+        }
+    }
+    ion = __any_sync(0xffffffffu, ion);
+    double S = block_exscan(acc, d.tot, tot);
+    if (tid == 0) {
+        d.xs[0] = tot;
+        d.xs[1] = rr[0];
+    }
+    dsync();  // totals published; Raman sub-transforms ready; field blocks no longer read
+    // the Raman polarisation of every block into tb (the field now lives in E); other CTAs write
+    // this one's, visible after the next barriers below
+    if (ir >= 0) raman_out_scatter<double, R>(d, d.tb, Mb);
+    for (int j = 0; j < q; ++j) S += drem(d.xs, j)[0];
+    const double y0r = drem(d.xs, 0)[1];
+    double fr[NS];
+    if (ion) {
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            S += rr[s];
+            const double f = dt * (S - 0.5 * (y0r + rr[s]));
+            fr[s] = pre1 - exp(-f);
+        }
+    } else {
+        const double f = dt * (S - 0.5 * y0r);
+        const double v = pre1 - ((f == 0.0) ? 1.0 : exp(-f));
+#pragma unroll
+        for (int s = 0; s < NS; ++s) fr[s] = v;
+    }
+    acc = 0;
+#pragma unroll
+    for (int s = 0; s < NS; ++s) acc += fr[s] * er * E[s];
+    double Tv = block_exscan(acc, d.tot + LUNA_WARPS, tot);
+    if (tid == 0) {
+        d.xs[2] = tot;
+        d.xs[3] = fr[0] * er * E[0];
+    }
+    dsync();
+    for (int j = 0; j < q; ++j) Tv += drem(d.xs, j)[2];
+    const double y0p = drem(d.xs, 0)[3];
+    // currents, in place of the rates
+    acc = 0;
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+        const double ph = fr[s] * er * E[s];
+        Tv += ph;
+        double J = dt * (Tv - 0.5 * (y0p + ph));
+        if (ion) J += (fabs(E[s]) > 0) ? ipot * rr[s] * (1.0 - fr[s]) / E[s] : 0.0;
+        rr[s] = J;
+        acc += J;
+    }
+    double U = block_exscan(acc, d.tot + 2 * LUNA_WARPS, tot);
+    if (tid == 0) {
+        d.xs[4] = tot;
+        d.xs[5] = rr[0];
+    }
+    dsync();
+    for (int j = 0; j < q; ++j) U += drem(d.xs, j)[4];
+    const double y0J = drem(d.xs, 0)[5];
+#pragma unroll
+    for (int h = 0; h < NS / 2; ++h) {
+        const int pos = Swz<double>::f(pr0 + h);
+        const cpx<double> rm = (ir >= 0) ? d.tb[pos] : mk<double>(0, 0);
+        const double2 tw = __ldg(reinterpret_cast<const double2*>(I.towin) + mbase + pr0 + h);
+        double P[2];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int s = 2 * h + c;
+            U += rr[s];
+            P[c] = kc * (E[s] * E[s] * E[s]) + coef * (dt * (U - 0.5 * (y0J + rr[s])));
+            if (ir >= 0) P[c] += rc * E[s] * (c ? rm.y : rm.x);
+        }
+        d.tb[pos] = mk<double>(P[0] * tw.x, P[1] * tw.y);
+    }
+    __syncthreads();
+}
+
 // ------------------------------------------------------------------ responses
 // Et_to_Pt! and the time window on this CTA's block (PlasmaScalar!, Nonlinear.jl:121-133,
 // as running trapezoids written as prefix sums; the carries into the block are the block
@@ -843,7 +941,15 @@ __device__ __noinline__ void dist_pointwise(const LunaInst& I, DWs<Rl>& d, int M
         __syncthreads();
         return;
     }
-    switch (2 * Mb / T) {  // samples per thread
+    if constexpr (sizeof(Rl) == 8) {
+        switch (2 * Mb / T) {  // samples per thread
+            case 2: dist_plasma_f64<2, R>(I, d, M, sc, ip, ir, kc, rc); break;
+            case 4: dist_plasma_f64<4, R>(I, d, M, sc, ip, ir, kc, rc); break;
+            case 8: dist_plasma_f64<8, R>(I, d, M, sc, ip, ir, kc, rc); break;
+            default: dist_plasma_f64<16, R>(I, d, M, sc, ip, ir, kc, rc); break;
+        }
+    } else
+    switch (2 * Mb / T) {
         case 4: dist_plasma<Rl, 4, R>(I, d, M, sc, ip, ir, kc, rc); break;
         case 8: dist_plasma<Rl, 8, R>(I, d, M, sc, ip, ir, kc, rc); break;
         default: dist_plasma<Rl, 16, R>(I, d, M, sc, ip, ir, kc, rc); break;

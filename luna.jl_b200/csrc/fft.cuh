@@ -127,11 +127,50 @@ __device__ __forceinline__ void apply_twiddles(cpx<R>* v, cpx<R> w) {
     }
 }
 
-// One in-place Stockham pass over a sub-transform of length Mb at `buf`; nact threads
-// are active, each with E/RAD butterflies.
-template <typename R, bool INV, int E, int RAD>
-__device__ __forceinline__ void pass_inplace(cpx<R>* buf, int Mb, int L, int nact, const TwTab<R>& tw) {
-    const int t = threadIdx.x;
+// Twiddle table of the shared-memory transforms in FP64: exp(-2 pi i a/4096), a < TWS_N, at
+// TWS_OFF of the CTA's dynamic shared memory (swizzled like the buffers). A radix-8 pass of span
+// L reads w = exp(-2 pi i k/(8 L)), entry k * 512/L, and w^2, and forms the other powers in one or
+// two products. Filled by every kernel that transforms (tws_fill); a pass then waits for shared
+// memory (~30 cycles) instead of L2 (~600 cycles, the L1 being what the buffers leave of 256 KB),
+// and its twiddles carry one to three roundings instead of three to seven (table product, then
+// powers). The FP32 transforms keep their tables in global memory: their pass radices, and so
+// their rounding, are those of the mixed-precision results.
+#define TWS_OFF 2048
+template <typename R> struct SmallBytes { static constexpr int v = 2048; };
+template <> struct SmallBytes<double> { static constexpr int v = TWS_OFF + TWS_N * 16; };
+
+template <typename R>
+__device__ __forceinline__ void tws_fill(const TwTab<R>& tw) {
+    if constexpr (sizeof(R) == 8) {
+        cpx<R>* t = reinterpret_cast<cpx<R>*>(dsm + TWS_OFF);
+        for (int a = threadIdx.x; a < TWS_N; a += LUNA_BLOCK)
+            t[Swz<R>::f(a)] = ldg(tw.fine + a);
+    }
+}
+template <typename R, bool INV>
+__device__ __forceinline__ cpx<R> tws_get(int a) {
+    const cpx<R> w = reinterpret_cast<const cpx<R>*>(dsm + TWS_OFF)[Swz<R>::f(a)];
+    return INV ? conj(w) : w;
+}
+
+// Multiply v[i] (bit-reversed slot i holds input r = bitrev(i)) by w^r, r = 1..7, from w and w^2.
+template <typename R>
+__device__ __forceinline__ void twiddle8(cpx<R>* v, cpx<R> w, cpx<R> w2) {
+    const cpx<R> w3 = w * w2, w4 = w2 * w2;
+    v[4] = v[4] * w;
+    v[2] = v[2] * w2;
+    v[6] = v[6] * w3;
+    v[1] = v[1] * w4;
+    v[5] = v[5] * (w * w4);
+    v[3] = v[3] * (w2 * w4);
+    v[7] = v[7] * (w3 * w4);
+}
+
+// One in-place Stockham pass over a sub-transform of length Mb at `buf`; the nact threads with
+// t < nact are active, each with E/RAD butterflies. TS: twiddles from the shared-memory table
+// (radix 8, L <= 512), else from global memory.
+template <typename R, bool INV, int E, int RAD, bool TS>
+__device__ __forceinline__ void pass_inplace(cpx<R>* buf, int Mb, int L, int nact, const TwTab<R>& tw, int t) {
     constexpr int NB = E / RAD;
     cpx<R> v[E];
     const int stride = Mb / RAD;
@@ -145,12 +184,17 @@ __device__ __forceinline__ void pass_inplace(cpx<R>* buf, int Mb, int L, int nac
     }
     __syncthreads();
     if (t < nact) {
-        const int shift = TW_LOG_MMAX - ilog2i((unsigned)(L * RAD));
+        const int lg = ilog2i((unsigned)(L * RAD));
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
             const int j = t + b * nact;
             const int k = j & (L - 1);
-            if (L > 1) apply_twiddles<R, RAD>(&v[b * RAD], twiddle<R, INV>(tw, (unsigned)k << shift));
+            if (L > 1) {
+                if constexpr (TS && RAD == 8) {
+                    const int a = k << (12 - lg);
+                    twiddle8<R>(&v[b * RAD], tws_get<R, INV>(a), tws_get<R, INV>(2 * a));
+                } else apply_twiddles<R, RAD>(&v[b * RAD], twiddle<R, INV>(tw, (unsigned)k << (TW_LOG_MMAX - lg)));
+            }
             dft_br<R, INV, RAD>(&v[b * RAD]);
             const int base = (j - k) * RAD + k;
 #pragma unroll
@@ -162,85 +206,21 @@ __device__ __forceinline__ void pass_inplace(cpx<R>* buf, int Mb, int L, int nac
 
 // In-place Stockham transform of one sub-block of length Mb = E * nact: a twiddle-free
 // first pass of the remainder radix, then passes of radix E.
-template <typename R, bool INV, int E>
-__device__ __forceinline__ void sub_fft(cpx<R>* buf, int Mb, const TwTab<R>& tw) {
+template <typename R, bool INV, int E, bool TS = false>
+__device__ __forceinline__ void sub_fft(cpx<R>* buf, int Mb, const TwTab<R>& tw, int t) {
     constexpr int LR = ilog2c<E>();
     const int nact = Mb / E;
     const int rem = ilog2i((unsigned)Mb) % LR;
     int L = 1;
     if (rem != 0) {
         const int r0 = 1 << rem;
-        if constexpr (E > 2) { if (r0 == 2) pass_inplace<R, INV, E, 2>(buf, Mb, 1, nact, tw); }
-        if constexpr (E > 4) { if (r0 == 4) pass_inplace<R, INV, E, 4>(buf, Mb, 1, nact, tw); }
-        if constexpr (E > 8) { if (r0 == 8) pass_inplace<R, INV, E, 8>(buf, Mb, 1, nact, tw); }
+        if constexpr (E > 2) { if (r0 == 2) pass_inplace<R, INV, E, 2, TS>(buf, Mb, 1, nact, tw, t); }
+        if constexpr (E > 4) { if (r0 == 4) pass_inplace<R, INV, E, 4, TS>(buf, Mb, 1, nact, tw, t); }
+        if constexpr (E > 8) { if (r0 == 8) pass_inplace<R, INV, E, 8, TS>(buf, Mb, 1, nact, tw, t); }
         L = r0;
     }
     while (L < Mb) {
-        pass_inplace<R, INV, E, E>(buf, Mb, L, nact, tw);
-        L *= E;
-    }
-}
-
-// The same transform of two buffers at once: one pass processes both, so the two
-// transforms share their barriers and twiddles (E/RAD butterflies per buffer and thread).
-template <typename R, bool INV, int E, int RAD>
-__device__ __forceinline__ void pass_inplace2(cpx<R>* ba, cpx<R>* bb, int Mb, int L, int nact, const TwTab<R>& tw) {
-    const int t = threadIdx.x;
-    constexpr int NB = E / RAD;
-    cpx<R> va[E], vb[E];
-    const int stride = Mb / RAD;
-    if (t < nact) {
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            const int j = t + b * nact;
-#pragma unroll
-            for (int i = 0; i < RAD; ++i) {
-                const int a = Swz<R>::f(j + bitrev<RAD>(i) * stride);
-                va[b * RAD + i] = ba[a];
-                vb[b * RAD + i] = bb[a];
-            }
-        }
-    }
-    __syncthreads();
-    if (t < nact) {
-        const int shift = TW_LOG_MMAX - ilog2i((unsigned)(L * RAD));
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            const int j = t + b * nact;
-            const int k = j & (L - 1);
-            if (L > 1) {
-                const cpx<R> w = twiddle<R, INV>(tw, (unsigned)k << shift);
-                apply_twiddles<R, RAD>(&va[b * RAD], w);
-                apply_twiddles<R, RAD>(&vb[b * RAD], w);
-            }
-            dft_br<R, INV, RAD>(&va[b * RAD]);
-            dft_br<R, INV, RAD>(&vb[b * RAD]);
-            const int base = (j - k) * RAD + k;
-#pragma unroll
-            for (int r = 0; r < RAD; ++r) {
-                const int a = Swz<R>::f(base + r * L);
-                ba[a] = va[b * RAD + r];
-                bb[a] = vb[b * RAD + r];
-            }
-        }
-    }
-    __syncthreads();
-}
-
-template <typename R, bool INV, int E>
-__device__ __forceinline__ void sub_fft2(cpx<R>* ba, cpx<R>* bb, int Mb, const TwTab<R>& tw) {
-    constexpr int LR = ilog2c<E>();
-    const int nact = Mb / E;
-    const int rem = ilog2i((unsigned)Mb) % LR;
-    int L = 1;
-    if (rem != 0) {
-        const int r0 = 1 << rem;
-        if constexpr (E > 2) { if (r0 == 2) pass_inplace2<R, INV, E, 2>(ba, bb, Mb, 1, nact, tw); }
-        if constexpr (E > 4) { if (r0 == 4) pass_inplace2<R, INV, E, 4>(ba, bb, Mb, 1, nact, tw); }
-        L = r0;
-    }
-    while (L < Mb) {
-        pass_inplace2<R, INV, E, E>(ba, bb, Mb, L, nact, tw);
+        pass_inplace<R, INV, E, E, TS>(buf, Mb, L, nact, tw, t);
         L *= E;
     }
 }
@@ -277,17 +257,73 @@ __device__ __forceinline__ void join_pass(cpx<R>* buf, int M, const TwTab<R>& tw
     __syncthreads();
 }
 
+// Passes over shared-memory buffers as functions of their own, given by the byte offset of the
+// buffer in the CTA's dynamic shared memory. What bounds a pass is latency (two barriers, a
+// twiddle lookup and shared-memory round trips at 8-16 active warps), so it must not also wait
+// for local memory or L2. Inlined into the solvers at their 128-register limit (64 in the FP32
+// column kernel), with every radix in one function, the passes spilled 600-2500 bytes a thread:
+// a 2048-point FP64 transform on 512 threads took 18-22 k cycles inside a right-hand side,
+// against 5.1 k alone as functions that keep a butterfly in registers, address shared memory
+// directly and (FP64) read their twiddles there; 9-12 k inside a right-hand side, where the
+// caller's registers are saved around them. The FP32 passes take the same radices, twiddles and
+// operations as before, so their results do not change.
+template <typename R>
+__device__ __forceinline__ unsigned dsm_off(const cpx<R>* p) {
+    return (unsigned)__cvta_generic_to_shared(p) - (unsigned)__cvta_generic_to_shared(dsm);
+}
+template <typename R>
+__device__ __forceinline__ cpx<R>* dsm_ptr(unsigned off) {
+    return reinterpret_cast<cpx<R>*>(dsm + off);
+}
+template <typename R, bool INV, int E, int RAD>
+__device__ __noinline__ void pass_s(unsigned off, int Mb, int L, int t, const TwTab<R> tw) {
+    pass_inplace<R, INV, E, RAD, sizeof(R) == 8>(dsm_ptr<R>(off), Mb, L, Mb / E, tw, t);
+}
+// sub_fft through pass_s
+template <typename R, bool INV, int E>
+__device__ __forceinline__ void sub_fft_s(unsigned off, int Mb, const TwTab<R>& tw, int t) {
+    constexpr int LR = ilog2c<E>();
+    const int rem = ilog2i((unsigned)Mb) % LR;
+    if constexpr (E > 2) { if (rem == 1) pass_s<R, INV, E, 2>(off, Mb, 1, t, tw); }
+    if constexpr (E > 4) { if (rem == 2) pass_s<R, INV, E, 4>(off, Mb, 1, t, tw); }
+    for (int L = 1 << rem; L < Mb; L *= E) pass_s<R, INV, E, E>(off, Mb, L, t, tw);
+}
+template <typename R, bool INV, int P>
+__device__ __noinline__ void join_pass_s(unsigned off, int M, const TwTab<R> tw) {
+    join_pass<R, INV, P>(dsm_ptr<R>(off), M, tw);
+}
+
+// One sub-transform of a cluster's CTA (natural order, in place, shared memory), in radix-8
+// passes (Mb/8 threads active): fewer barrier-separated passes matter more than idle threads.
 template <typename R, bool INV>
-__device__ __forceinline__ void sub_ffts(cpx<R>* buf, int M, int P, const TwTab<R>& tw) {
+__device__ __forceinline__ void fft_sub1(cpx<R>* b, int Mb, const TwTab<R>& tw) {
+    sub_fft_s<R, INV, 8>(dsm_off(b), Mb, tw, threadIdx.x);
+}
+// Two of them: by the two halves of the CTA where a half holds a pass (Mb <= 8 * LUNA_BLOCK/2),
+// which share the barriers while a thread keeps one butterfly in registers (both buffers'
+// butterflies in every thread spilled 1.3 kB in FP64), else one after the other.
+template <typename R, bool INV>
+__device__ __forceinline__ void fft_sub2(cpx<R>* ba, cpx<R>* bb, int Mb, const TwTab<R>& tw) {
+    constexpr int H = LUNA_BLOCK / 2;
+    if (Mb <= 8 * H) {
+        sub_fft_s<R, INV, 8>(dsm_off(threadIdx.x < H ? ba : bb), Mb, tw, threadIdx.x & (H - 1));
+    } else {
+        sub_fft_s<R, INV, 8>(dsm_off(ba), Mb, tw, threadIdx.x);
+        sub_fft_s<R, INV, 8>(dsm_off(bb), Mb, tw, threadIdx.x);
+    }
+}
+
+// The P sub-transforms of a buffer in shared memory. FP64 takes radix-8 passes at every length
+// (512 to 4096 points take as long with all 512 threads in radix-2 and radix-4 passes, and one
+// code path stays in the instruction cache); FP32 the radix that keeps every thread busy.
+template <typename R, bool INV>
+__device__ __forceinline__ void sub_ffts(unsigned off, int M, int P, const TwTab<R>& tw) {
     const int Mb = M / P;
-    int E = Mb / LUNA_BLOCK;
-    if (E < 2) E = 2;
-    for (int p = 0; p < P; ++p) {
-        cpx<R>* b = buf + (size_t)p * Mb;
-        if (E == 2) sub_fft<R, INV, 2>(b, Mb, tw);
-        else if (E == 4) sub_fft<R, INV, 4>(b, Mb, tw);
-        else if (E == 8) sub_fft<R, INV, 8>(b, Mb, tw);
-        else if constexpr (FftEmax<R>::v >= 16) sub_fft<R, INV, 16>(b, Mb, tw);
+    const int E = (sizeof(R) == 8) ? 8 : Mb / LUNA_BLOCK;
+    for (int p = 0; p < P; ++p, off += (unsigned)(Mb * sizeof(cpx<R>))) {
+        if (E == 8) sub_fft_s<R, INV, 8>(off, Mb, tw, threadIdx.x);
+        else if (E == 4) sub_fft_s<R, INV, 4>(off, Mb, tw, threadIdx.x);
+        else sub_fft_s<R, INV, 2>(off, Mb, tw, threadIdx.x);
     }
 }
 
@@ -352,19 +388,26 @@ __device__ __forceinline__ int split_pos(int n, int M, int P) {
 }
 
 // Unnormalised DFT of length M (power of two, 2 <= M <= FftMmax).
-// With alt == nullptr (shared-memory buffers) it runs in place:
+// With alt == nullptr the buffer is in the dynamic shared memory and it runs in place:
 //   forward (INV=false): split-order input -> natural-order output
 //   inverse (INV=true):  natural-order input -> split-order output
 // With a second buffer alt (global-memory buffers) it runs out of place in natural order
 // both ways. Returns the buffer holding the result. The caller synchronises before the
 // call (the input is written by other threads); the call ends with a barrier.
 template <typename R, bool INV>
-__device__ __forceinline__ void block_fft_split(cpx<R>* buf, int M, const TwTab<R>& tw);
-
+__device__ __noinline__ cpx<R>* fft_oop_g(cpx<R>* buf, cpx<R>* alt, int M, const TwTab<R> tw) {
+    return fft_oop<R, INV>(buf, alt, M, tw);
+}
 template <typename R, bool INV>
-__device__ __noinline__ cpx<R>* block_fft(cpx<R>* buf, cpx<R>* alt, int M, const TwTab<R>& tw) {
-    if (alt) return fft_oop<R, INV>(buf, alt, M, tw);
-    block_fft_split<R, INV>(buf, M, tw);
+__device__ __forceinline__ cpx<R>* block_fft(cpx<R>* buf, cpx<R>* alt, int M, const TwTab<R>& tw) {
+    if (alt) return fft_oop_g<R, INV>(buf, alt, M, tw);
+    const int P = fft_nsplit<R>(M);
+    const unsigned off = dsm_off(buf);
+    if (!INV) sub_ffts<R, INV>(off, M, P, tw);
+    if (P == 2) join_pass_s<R, INV, 2>(off, M, tw);
+    else if (P == 4) join_pass_s<R, INV, 4>(off, M, tw);
+    else if (P == 8) join_pass_s<R, INV, 8>(off, M, tw);
+    if (INV) sub_ffts<R, INV>(off, M, P, tw);
     return buf;
 }
 
@@ -374,20 +417,14 @@ __device__ __forceinline__ int buf_split(const cpx<R>* alt, int M) {
     return alt ? 1 : fft_nsplit<R>(M);
 }
 
-template <typename R, bool INV>
-__device__ __forceinline__ void block_fft_split(cpx<R>* buf, int M, const TwTab<R>& tw) {
-    const int P = fft_nsplit<R>(M);
-    if (INV) {
-        if (P == 2) join_pass<R, INV, 2>(buf, M, tw);
-        else if (P == 4) join_pass<R, INV, 4>(buf, M, tw);
-        else if (P == 8) join_pass<R, INV, 8>(buf, M, tw);
-        sub_ffts<R, INV>(buf, M, P, tw);
-    } else {
-        sub_ffts<R, INV>(buf, M, P, tw);
-        if (P == 2) join_pass<R, INV, 2>(buf, M, tw);
-        else if (P == 4) join_pass<R, INV, 4>(buf, M, tw);
-        else if (P == 8) join_pass<R, INV, 8>(buf, M, tw);
-    }
+// The forward transform of block_fft on one FP64 buffer in global memory (split-order input,
+// natural output, in place): plan creation only.
+__device__ __forceinline__ void fft_fwd_inplace(cpx<double>* buf, int M, const TwTab<double>& tw) {
+    const int P = fft_nsplit<double>(M), Mb = M / P;
+    for (int p = 0; p < P; ++p) sub_fft<double, false, 8>(buf + (size_t)p * Mb, Mb, tw, threadIdx.x);
+    if (P == 2) join_pass<double, false, 2>(buf, M, tw);
+    else if (P == 4) join_pass<double, false, 4>(buf, M, tw);
+    else if (P == 8) join_pass<double, false, 8>(buf, M, tw);
 }
 
 }  // namespace luna

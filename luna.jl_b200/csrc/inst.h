@@ -27,6 +27,7 @@ typedef struct {
     const double* sx;
     const double* sy;
     const double* sD;
+    const double2* spk;  // the same nodes packed as (x, y), (D, 0): FP64 plans
     const float* sxf;
     const float* syf;
     const float* sDf;

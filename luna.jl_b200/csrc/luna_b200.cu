@@ -28,16 +28,19 @@ using namespace luna;
 template <typename Rl, typename Kt>
 __global__ void __launch_bounds__(LUNA_BLOCK, 1)
 solve_kernel(LunaInst* insts, int n, int* counter, TwTab<Rl> tw, int smem_bytes, const int* list) {
-    extern __shared__ __align__(256) char smem[];
+    char* const smem = dsm;
     __shared__ Ctl ctl;
     __shared__ int sidx;
+    __shared__ LunaInst sI;
+    tws_fill(tw);
     while (true) {
         __syncthreads();
         if (threadIdx.x == 0) sidx = atomicAdd(counter, 1);
         __syncthreads();
         const int q = sidx;
         if (q >= n) break;
-        LunaInst& I = insts[list ? list[q] : q];
+        LunaInst* gI = insts + (list ? list[q] : q);
+        LunaInst& I = local_inst<Rl>(gI, &sI);
         if (threadIdx.x == 0) {
             unsigned long long t;
             unsigned int sm;
@@ -54,6 +57,7 @@ solve_kernel(LunaInst* insts, int n, int* counter, TwTab<Rl> tw, int smem_bytes,
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
             I.t_end = t;
         }
+        return_inst<Rl>(gI, &sI);
     }
 }
 
@@ -72,7 +76,7 @@ __device__ void cluster_helper(LunaInst* insts, char* smem, int smem_bytes, cons
                                ClBox* box, int* err) {
     namespace cg = cooperative_groups;
     const int tid = threadIdx.x, T = LUNA_BLOCK;
-    cpx<Rl>* buf = reinterpret_cast<cpx<Rl>*>(smem + LUNA_SMALL_BYTES);
+    cpx<Rl>* buf = reinterpret_cast<cpx<Rl>*>(smem + SmallBytes<Rl>::v);
     __shared__ int s_ok;
     int seen = 0;
     const int par = (int)rank - 1;
@@ -207,7 +211,7 @@ __global__ void __launch_bounds__(LUNA_BLOCK, 1)
 solve_kernel_cl(LunaInst* insts, const int* big, int nbig, int* big_counter, const int* reg, int nreg,
                 int* reg_counter, TwTab<Rl> tw, int smem_bytes, int* err) {
     namespace cg = cooperative_groups;
-    extern __shared__ __align__(256) char smem[];
+    char* const smem = dsm;
     __shared__ Ctl ctl;
     __shared__ ClBox box;
     __shared__ int sidx;
@@ -243,9 +247,9 @@ solve_kernel_cl(LunaInst* insts, const int* big, int nbig, int* big_counter, con
             Ws<Rl> w;
             plan_ws<Rl>(I, smem, smem_bytes, w, tw, nullptr, true);
             w.cl = &box;
-            w.rem_e = cl.map_shared_rank(reinterpret_cast<cpx<Rl>*>(smem + LUNA_SMALL_BYTES), 1);
-            w.rem_o = cl.map_shared_rank(reinterpret_cast<cpx<Rl>*>(smem + LUNA_SMALL_BYTES), 2);
-            w.rem_p = cl.map_shared_rank(reinterpret_cast<cpx<Rl>*>(smem + LUNA_SMALL_BYTES), 3);
+            w.rem_e = cl.map_shared_rank(reinterpret_cast<cpx<Rl>*>(smem + SmallBytes<Rl>::v), 1);
+            w.rem_o = cl.map_shared_rank(reinterpret_cast<cpx<Rl>*>(smem + SmallBytes<Rl>::v), 2);
+            w.rem_p = cl.map_shared_rank(reinterpret_cast<cpx<Rl>*>(smem + SmallBytes<Rl>::v), 3);
             solve_instance<Rl, Kt>(I, w, ctl);
             if (threadIdx.x == 0) {
                 unsigned long long t;
@@ -300,18 +304,21 @@ __global__ void __launch_bounds__(LUNA_BLOCK, 1)
 solve_kernel_dist(LunaInst* insts, const int* dl, int nd, int* d_counter, const int* reg, int nreg,
                   int* reg_counter, TwTab<Rl> tw, int smem_bytes) {
     namespace cg = cooperative_groups;
-    extern __shared__ __align__(256) char smem[];
+    char* const smem = dsm;
     __shared__ Ctl ctl;
     __shared__ int sidx;
+    __shared__ LunaInst sI;  // FP64: every CTA of the cluster has its copy; rank 0 writes the results back
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank();
+    tws_fill(tw);
     while (true) {
         if (rank == 0 && threadIdx.x == 0) sidx = atomicAdd(d_counter, 1);
         cl.sync();
         const int q = *cl.map_shared_rank(&sidx, 0);
         cl.sync();  // rank 0's index is read everywhere before the next pull overwrites it
         if (q >= nd) break;
-        LunaInst& I = insts[dl[q]];
+        LunaInst* gI = insts + dl[q];
+        LunaInst& I = local_inst<Rl>(gI, &sI);
         if (rank == 0 && threadIdx.x == 0) {
             unsigned long long t;
             unsigned int sm;
@@ -328,6 +335,7 @@ solve_kernel_dist(LunaInst* insts, const int* dl, int nd, int* d_counter, const 
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
             I.t_end = t;
         }
+        if (rank == 0) return_inst<Rl>(gI, &sI);
     }
     while (true) {
         __syncthreads();
@@ -335,7 +343,8 @@ solve_kernel_dist(LunaInst* insts, const int* dl, int nd, int* d_counter, const 
         __syncthreads();
         const int q = sidx;
         if (q >= nreg) break;
-        LunaInst& I = insts[reg[q]];
+        LunaInst* gI = insts + reg[q];
+        LunaInst& I = local_inst<Rl>(gI, &sI);
         if (threadIdx.x == 0) {
             unsigned long long t;
             unsigned int sm;
@@ -352,6 +361,7 @@ solve_kernel_dist(LunaInst* insts, const int* dl, int nd, int* d_counter, const 
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
             I.t_end = t;
         }
+        return_inst<Rl>(gI, &sI);
     }
 }
 
@@ -359,8 +369,10 @@ solve_kernel_dist(LunaInst* insts, const int* dl, int nd, int* d_counter, const 
 template <typename Rl>
 __global__ void __launch_bounds__(LUNA_BLOCK, 1)
 rhs_kernel(LunaInst* inst, const double2* Ew, double2* nl, TwTab<Rl> tw, int smem_bytes, int* status, double z) {
-    extern __shared__ __align__(256) char smem[];
-    LunaInst& I = *inst;
+    char* const smem = dsm;
+    __shared__ LunaInst sI;
+    tws_fill(tw);
+    LunaInst& I = local_inst<Rl>(inst, &sI);
     Ws<Rl> w;
     plan_ws<Rl>(I, smem, smem_bytes, w, tw);
     if (threadIdx.x == 0) *w.flag = 0;
@@ -399,7 +411,8 @@ raman_h_kernel(LunaResp r, int No, double hscale, cpx<double>* buf, cpx<Rl>* H, 
         buf[Swz<double>::f(split_pos(m, No, P))] = mk<double>(a, b);
     }
     __syncthreads();
-    cpx<double>* Z = block_fft<double, false>(buf, nullptr, No, tw);
+    fft_fwd_inplace(buf, No, tw);
+    const cpx<double>* Z = buf;
     const int M = No;
     for (int k = tid; k <= M; k += LUNA_BLOCK) {
         const int kk = k & (M - 1);
@@ -464,8 +477,17 @@ int get_tw(TwDev& out) {
         hi[j] = mk<double>(std::cos(a), std::sin(a));
         hif[j] = mk<float>((float)hi[j].x, (float)hi[j].y);
     }
+    std::vector<cpx<double>> fine(TWS_N);
+    for (int j = 0; j < TWS_N; ++j) {
+        double a = -two_pi * (double)j / 4096.0;
+        fine[j] = mk<double>(std::cos(a), std::sin(a));
+    }
     TwDev t;
     void* p;
+    CK(cudaMalloc(&p, sizeof(cpx<double>) * TWS_N));
+    CK(cudaMemcpy(p, fine.data(), sizeof(cpx<double>) * TWS_N, cudaMemcpyHostToDevice));
+    t.d.fine = (const cpx<double>*)p;
+    t.f.fine = nullptr;
     CK(cudaMalloc(&p, sizeof(cpx<double>) * (TW_NLO + TW_NHI)));
     CK(cudaMemcpy(p, lo.data(), sizeof(cpx<double>) * TW_NLO, cudaMemcpyHostToDevice));
     CK(cudaMemcpy((char*)p + sizeof(cpx<double>) * TW_NLO, hi.data(), sizeof(cpx<double>) * TW_NHI,
@@ -489,13 +511,13 @@ int max_smem_optin() {
     int dev = 0, v = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    return v - 1024;  // leave room for the kernels' static shared memory
+    return v - 3072;  // leave room for the kernels' static shared memory
 }
 
 template <typename Rl>
 size_t smem_wanted(const LunaInst& I) {
     const size_t c = sizeof(cpx<Rl>);
-    size_t s = LUNA_SMALL_BYTES;
+    size_t s = SmallBytes<Rl>::v;
     s += align_up((size_t)main_len(I) * c, 256);
     if (needs_hilbert(I)) s += align_up((size_t)(I.No / 2) * c, 256);
     s += align_up((size_t)I.Nw * c, 256);
@@ -867,6 +889,22 @@ int luna_b200_plan_create(const luna_grid_desc* g, const luna_resp_desc* resps, 
                     UP(d.spl_x, d.spl_n, &r.sx);
                     UP(d.spl_y, d.spl_n, &r.sy);
                     UP(d.spl_D, d.spl_n, &r.sD);
+                    if (precision == LUNA_PREC_FP64) {
+                        std::vector<double> pk(4 * (size_t)d.spl_n);
+                        for (int j = 0; j < d.spl_n; ++j) {
+                            pk[4 * (size_t)j] = d.spl_x[j];
+                            pk[4 * (size_t)j + 1] = d.spl_y[j];
+                            pk[4 * (size_t)j + 2] = d.spl_D[j];
+                            pk[4 * (size_t)j + 3] = 0.0;
+                        }
+                        const double* t = nullptr;
+                        UP(pk.data(), pk.size(), &t);
+                        r.spk = reinterpret_cast<const double2*>(t);
+                        r.sn = d.spl_n;
+                        r.Emin = d.spl_x[0];
+                        r.Emax = d.spl_x[d.spl_n - 1];
+                        break;
+                    }
                     std::vector<float> fx(d.spl_n), fy(d.spl_n), fD(d.spl_n);
                     for (int j = 0; j < d.spl_n; ++j) {
                         fx[j] = (float)d.spl_x[j];
@@ -1258,7 +1296,7 @@ int luna_b200_batch_create(luna_plan* const* plans, int n, const luna_solve_opts
             const size_t efac = align_up((size_t)I.Nw * sizeof(float2), 256);
             const bool fits1 = smem_wanted<float>(I) <= (size_t)maxs;
             const bool ok_cl = I.kind == 0 && has_raman(I) && !fits1 && !needs_hilbert(I) && !I.grad &&
-                               LUNA_SMALL_BYTES + half + efac <= (size_t)std::min<int>(maxs, b->smem);
+                               SmallBytes<float>::v + half + efac <= (size_t)std::min<int>(maxs, b->smem);
             if (ok_cl) big.push_back(i);
             else reg.push_back(i);
             cost[i] = (double)I.No * std::log2((double)I.No) * (has_raman(I) ? 2.0 : 1.0);
@@ -2131,7 +2169,7 @@ int modal_setup(luna_modal_plan* p) {
     }
     // split factor of the time buffers: the block transform's when the buffer is in shared
     // memory (the same test as plan_ws), natural order otherwise
-    const bool main_smem = LUNA_SMALL_BYTES + align_up((size_t)M * sizeof(cpx<Rl>), 256) <= (size_t)p->smem;
+    const bool main_smem = SmallBytes<Rl>::v + align_up((size_t)M * sizeof(cpx<Rl>), 256) <= (size_t)p->smem;
     p->P = main_smem ? fft_nsplit<Rl>(M) : 1;
     p->nchunk = std::max(1, std::min(M / 256, 4 * 148));
     if (dalloc(p->allocs, &p->Et, sizeof(cpx<Rl>) * (size_t)p->Nr * M) ||
@@ -2350,7 +2388,8 @@ static_assert(ST_OK == LUNA_OK && ST_FIELD_ABOVE_EMAX == LUNA_FIELD_ABOVE_EMAX,
 template <typename Rl>
 __global__ void __launch_bounds__(LUNA_BLOCK, 1)
 rhs_kernel_noalloc(const LunaInst I, const double2* Ew, double2* nl, TwTab<Rl> tw, int smem_bytes, int* status) {
-    extern __shared__ __align__(256) char smem[];
+    char* const smem = dsm;
+    tws_fill(tw);
     Ws<Rl> w;
     plan_ws<Rl>(I, smem, smem_bytes, w, tw);
     if (threadIdx.x == 0) *w.flag = 0;

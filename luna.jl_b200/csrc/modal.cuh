@@ -63,9 +63,11 @@ template <typename Rl>
 __global__ void __launch_bounds__(LUNA_BLOCK, 1)
 modal_time_kernel(const LunaInst* inst, const cpx<Rl>* A, ModalArgs a, TwTab<Rl> tw, int smem_bytes,
                   char* gscr, size_t gstride) {
-    extern __shared__ __align__(256) char smem[];
+    char* const smem = dsm;
     if (a.st && a.st->finished) return;
-    const LunaInst& I = *inst;
+    __shared__ LunaInst sI;
+    tws_fill(tw);
+    const LunaInst& I = local_inst<Rl>(inst, &sI);
     const int c = blockIdx.x;
     if (c == 0 && threadIdx.x == 0) {
         a.ms->done = 0;
@@ -91,9 +93,11 @@ template <typename Rl>
 __global__ void __launch_bounds__(LUNA_BLOCK, 1)
 modal_node_kernel(const LunaInst* inst, ModalArgs a, int slot0, TwTab<Rl> tw, int smem_bytes, char* gscr,
                   size_t gstride, int* flags) {
-    extern __shared__ __align__(256) char smem[];
+    char* const smem = dsm;
     if (modal_skip(a)) return;
-    const LunaInst& I = *inst;
+    __shared__ LunaInst sI;
+    tws_fill(tw);
+    const LunaInst& I = local_inst<Rl>(inst, &sI);
     const int slot = slot0 + blockIdx.x;
     Ws<Rl> w;
     plan_ws<Rl>(I, smem, smem_bytes, w, tw, gscr ? gscr + (size_t)blockIdx.x * gstride : nullptr);
@@ -341,9 +345,11 @@ template <typename Rl>
 __global__ void __launch_bounds__(LUNA_BLOCK, 1)
 modal_level_kernel(const LunaInst* inst, ModalArgs a, int l, cpx<Rl>* B, TwTab<Rl> tw, int smem_bytes,
                    char* gscr, size_t gstride) {
-    extern __shared__ __align__(256) char smem[];
+    char* const smem = dsm;
     if (modal_skip(a)) return;
-    const LunaInst& I = *inst;
+    __shared__ LunaInst sI;
+    tws_fill(tw);
+    const LunaInst& I = local_inst<Rl>(inst, &sI);
     const int c = blockIdx.x;
     Ws<Rl> w;
     plan_ws<Rl>(I, smem, smem_bytes, w, tw, gscr ? gscr + (size_t)c * gstride : nullptr);

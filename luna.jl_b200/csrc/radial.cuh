@@ -276,9 +276,11 @@ template <typename Rl>
 __global__ void __launch_bounds__(LUNA_BLOCK, sizeof(Rl) == 4 ? 2 : 1)
 rad_column_kernel(const LunaInst* inst, const cpx<Rl>* Er, cpx<Rl>* Pw, TwTab<Rl> tw, int smem_bytes,
                   char* gscr, size_t gstride, RadState* st, int* flags) {
-    extern __shared__ __align__(256) char smem[];
+    char* const smem = dsm;
     if (st && st->finished) return;
-    const LunaInst& I = *inst;
+    __shared__ LunaInst sI;
+    tws_fill(tw);
+    const LunaInst& I = local_inst<Rl>(inst, &sI);
     const int c = blockIdx.x;
     Ws<Rl> w;
     plan_ws<Rl>(I, smem, smem_bytes, w, tw, gscr ? gscr + (size_t)c * gstride : nullptr);
@@ -449,10 +451,12 @@ template <typename Rl, typename Kt>
 __global__ void __launch_bounds__(LUNA_BLOCK, 1)
 rad_post_kernel(RadArgs a, const LunaInst* inst, const LunaInst* opt, TwTab<Rl> tw, int smem_bytes, char* gscr,
                 size_t gstride, RadGrad G) {
-    extern __shared__ __align__(256) char smem[];
+    char* const smem = dsm;
     const RadState* st = a.st;
     if (st->finished) return;
-    const LunaInst& I = *inst;
+    __shared__ LunaInst sI;
+    tws_fill(tw);
+    const LunaInst& I = local_inst<Rl>(inst, &sI);
     const int c = blockIdx.x, Nw = a.Nw;
     const size_t off = (size_t)c * Nw;
     double2* y = st->y + off;

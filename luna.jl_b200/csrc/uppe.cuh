@@ -74,6 +74,35 @@ struct Ctl {  // controller state shared by the CTA (shared memory)
 
 __host__ __device__ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
+// FP64 kernels work on a copy of their instance description in shared memory (every field is
+// read many times, by chains of dependent loads; from L2 the buffer layout alone took 3.7 k
+// cycles): local_inst copies it with the whole CTA, return_inst writes it back after a solve.
+static_assert(sizeof(LunaInst) % 8 == 0, "LunaInst is copied in 8-byte words");
+__device__ __forceinline__ void copy_inst(LunaInst* dst, const LunaInst* src) {
+    __syncthreads();
+    const unsigned long long* s = reinterpret_cast<const unsigned long long*>(src);
+    unsigned long long* d = reinterpret_cast<unsigned long long*>(dst);
+    for (int i = threadIdx.x; i < (int)(sizeof(LunaInst) / 8); i += LUNA_BLOCK) d[i] = s[i];
+    __syncthreads();
+}
+template <typename Rl>
+__device__ __forceinline__ LunaInst& local_inst(LunaInst* g, LunaInst* sh) {
+    if constexpr (sizeof(Rl) == 8) {
+        copy_inst(sh, g);
+        return *sh;
+    } else {
+        return *g;
+    }
+}
+template <typename Rl>
+__device__ __forceinline__ const LunaInst& local_inst(const LunaInst* g, LunaInst* sh) {
+    return local_inst<Rl>(const_cast<LunaInst*>(g), sh);
+}
+template <typename Rl>
+__device__ __forceinline__ void return_inst(LunaInst* g, const LunaInst* sh) {
+    if constexpr (sizeof(Rl) == 8) copy_inst(g, sh);
+}
+
 // main transform length (complex elements) for an instance
 __host__ __device__ inline int main_len(const LunaInst& I) {
     int M = (I.kind == 0) ? I.No / 2 : I.No;
@@ -112,8 +141,6 @@ __host__ __device__ inline size_t gscr_bytes(const LunaInst& I) {
     return b;
 }
 
-#define LUNA_SMALL_BYTES 2048
-
 template <typename Rl>
 __device__ void plan_ws(const LunaInst& I, char* smem, int smem_bytes, Ws<Rl>& w, const TwTab<Rl>& tw,
                         void* gscr = nullptr, bool raman_remote = false) {
@@ -124,7 +151,7 @@ __device__ void plan_ws(const LunaInst& I, char* smem, int smem_bytes, Ws<Rl>& w
     w.edge = w.tot + 3 * LUNA_WARPS;
     w.flag = reinterpret_cast<int*>(w.edge + 4);
     w.tw = tw;
-    size_t off = LUNA_SMALL_BYTES;
+    size_t off = SmallBytes<Rl>::v;
     const size_t c = sizeof(cpx<Rl>);
     char* g = reinterpret_cast<char*>(gscr ? gscr : I.gscr);
     size_t goff = 0;
@@ -303,6 +330,65 @@ __device__ __forceinline__ Rl adk_rate(const LunaResp& r, Rl aE) {
 template <typename Rl>
 __device__ __forceinline__ Rl eval_rate(const LunaResp& r, Rl aE, int* flag) {
     return r.kind == LUNA_RESP_PLASMA_PPT ? ppt_rate<Rl>(r, aE, flag) : adk_rate<Rl>(r, aE);
+}
+
+// Rates of NS samples in FP64 (NaN fields give NaN, fields above the table raise the flag, as in
+// ppt_rate<double> / adk_rate<double>). What bounds the rates is latency: the two table nodes of
+// a sample come from L2, a division and exp follow, and taken one after the other with their
+// early exits four samples cost ~5 k cycles. Here a warp without a field in range leaves at
+// once (nearly all of the time window), and otherwise the NS samples are evaluated without
+// branches, their loads and divisions in flight together; a node's (x, y, D) sits in one 32-byte
+// sector. The ADK form takes exp(pw log(a/|E|) - b/|E|), one logarithm instead of pow.
+// Call with whole warps.
+template <int NS>
+__device__ __forceinline__ void rates_f64(const LunaResp& r, const double* E, int* flag, double* out) {
+    bool in[NS], any = false;
+    double aE[NS];
+    const bool ppt = r.kind == LUNA_RESP_PLASMA_PPT;
+    const double lo = ppt ? r.Emin : r.adk_thr;
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+        aE[s] = fabs(E[s]);
+        in[s] = !(aE[s] < lo) && aE[s] != 0.0;
+        out[s] = 0.0;
+        any = any || in[s];
+    }
+    if (!__any_sync(0xffffffffu, any)) return;
+    if (ppt) {
+        const double xmin = r.Emin, xmax = r.Emax, n1 = (double)(r.sn - 1), q = n1 / (xmax - xmin);
+        double2 a[NS], b[NS];
+        double Da[NS], Db[NS];
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            const int i = (int)fmin(fmax(ceil((aE[s] - xmin) * q), 1.0), n1);  // node above, 1..sn-1
+            const double2* t = r.spk + 2 * (size_t)i;
+            a[s] = __ldg(t - 2);
+            Da[s] = __ldg(&t[-1].x);
+            b[s] = __ldg(t);
+            Db[s] = __ldg(&t[1].x);
+        }
+        bool above = false;
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            const double t = (aE[s] - a[s].x) / (b[s].x - a[s].x);
+            double v = a[s].y + Da[s] * t + (3.0 * (b[s].y - a[s].y) - 2.0 * Da[s] - Db[s]) * (t * t)
+                       + (2.0 * (a[s].y - b[s].y) + Da[s] + Db[s]) * (t * t * t);
+            v = (aE[s] == b[s].x) ? b[s].y : (aE[s] == a[s].x) ? a[s].y : v;
+            const bool ab = aE[s] > xmax;
+            above = above || ab;
+            const double e = exp(v);
+            out[s] = (in[s] && !ab) ? e : 0.0;
+        }
+        if (above) atomicOr(flag, 1 << ST_FIELD_ABOVE_EMAX);
+    } else {
+        const double pa = r.adk_a, pb = r.adk_b, pw = r.adk_pw, pre = r.adk_pre;
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            const double ix = 1.0 / aE[s];
+            const double e = pre * exp(pw * log(pa * ix) - pb * ix);
+            out[s] = in[s] ? e : 0.0;
+        }
+    }
 }
 
 // ------------------------------------------------------------------ real-FFT helpers
@@ -550,6 +636,107 @@ __device__ __forceinline__ void plasma_quad(const LunaResp& r, const bool act[2]
     }
 }
 
+// PlasmaScalar! (Nonlinear.jl:121-133) with Kerr, Raman and the time window in FP64 on the M
+// sample pairs of x, NP consecutive pairs per thread and chunk: the three running trapezoids
+// of plasma_quad as block prefix sums of 2 NP samples a thread. Bound by latency (three block
+// scans a chunk at 16 warps), so a chunk is as long as the registers allow (2048 pairs), and the
+// transcendental work is left out where it has no effect: without ionisation in a thread's
+// samples its fraction is one value (one exp instead of 2 NP) and its loss current zero.
+template <int NP>
+__device__ __noinline__ void plasma_real_f64(const LunaInst& I, Ws<double>& w, cpx<double>* x, int M, int P, double sc,
+                                             int ip, int ir, const cpx<double>* Pr, int Pr_split) {
+    constexpr int NS = 2 * NP;
+    const int T = LUNA_BLOCK, tid = threadIdx.x;
+    const LunaResp& r = I.resp[ip];
+    const double dt = r.dt, er = r.eratio, coef = r.coef, ipot = r.ionpot, pre1 = r.preion + 1.0;
+    double kc = 0, rc = 0;
+    for (int i = 0; i < I.nresp; ++i) {
+        if (I.resp[i].kind == LUNA_RESP_KERR_FIELD) kc += I.resp[i].coef;
+        if (i == ir) rc = I.resp[i].coef;
+    }
+    double c1 = 0, c2 = 0, c3 = 0, tot;
+    for (int c0 = 0; c0 < M; c0 += NP * T) {
+        const int m0 = c0 + NP * tid;
+        double E[NS], rr[NS], fr[NS];
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+            const cpx<double> e = x[Swz<double>::f(split_pos(m0 + q, M, P))];
+            E[2 * q] = e.x * sc;
+            E[2 * q + 1] = e.y * sc;
+        }
+        rates_f64<NS>(r, E, w.flag, rr);
+        if (m0 == 0) w.edge[0] = rr[0];
+        double acc = 0;
+        bool ion = false;
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            acc += rr[s];
+            ion = ion || rr[s] != 0.0;
+        }
+        ion = __any_sync(0xffffffffu, ion);
+        double S = c1 + block_exscan(acc, w.tot, tot);
+        c1 += tot;
+        const double y0r = w.edge[0];
+        if (ion) {
+#pragma unroll
+            for (int s = 0; s < NS; ++s) {
+                S += rr[s];
+                const double f = dt * (S - 0.5 * (y0r + rr[s]));
+                fr[s] = pre1 - exp(-f);
+            }
+        } else {
+            const double f = dt * (S - 0.5 * y0r);
+            const double v = pre1 - ((f == 0.0) ? 1.0 : exp(-f));
+#pragma unroll
+            for (int s = 0; s < NS; ++s) fr[s] = v;
+        }
+        acc = 0;
+#pragma unroll
+        for (int s = 0; s < NS; ++s) acc += fr[s] * er * E[s];
+        if (m0 == 0) w.edge[1] = fr[0] * er * E[0];
+        double Tv = c2 + block_exscan(acc, w.tot + LUNA_WARPS, tot);
+        c2 += tot;
+        const double y0p = w.edge[1];
+        acc = 0;
+        double J[NS];
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            const double ph = fr[s] * er * E[s];
+            Tv += ph;
+            J[s] = dt * (Tv - 0.5 * (y0p + ph));
+        }
+        if (ion) {
+#pragma unroll
+            for (int s = 0; s < NS; ++s)
+                J[s] += (fabs(E[s]) > 0) ? ipot * rr[s] * (1.0 - fr[s]) / E[s] : 0.0;
+        }
+#pragma unroll
+        for (int s = 0; s < NS; ++s) acc += J[s];
+        if (m0 == 0) w.edge[2] = J[0];
+        double U = c3 + block_exscan(acc, w.tot + 2 * LUNA_WARPS, tot);
+        c3 += tot;
+        const double y0J = w.edge[2];
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+            const int m = m0 + q;
+            cpx<double> pr = mk<double>(0, 0);
+            if (ir >= 0) pr = Pr[Swz<double>::f(split_pos(m, I.No, Pr_split))];
+            const double2 tw = __ldg(reinterpret_cast<const double2*>(I.towin) + m);
+            double p[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int s = 2 * q + h;
+                const double Es = E[s];
+                U += J[s];
+                p[h] = kc * (Es * Es * Es) + coef * (dt * (U - 0.5 * (y0J + J[s])));
+                if (ir >= 0) p[h] += rc * Es * (h ? pr.y : pr.x);
+            }
+            x[Swz<double>::f(split_pos(m, M, P))] = mk<double>(p[0] * tw.x, p[1] * tw.y);
+        }
+    }
+    __syncthreads();
+}
+
 // Plasma polarisation alone, for the plasma helper of a response cluster: the field is
 // read from xr (rank 0's buffer, split factor P) and rho * P_plasma is written to out at
 // the same positions.
@@ -738,6 +925,14 @@ __device__ __forceinline__ void pointwise_real_t(const LunaInst& I, Ws<Rl>& w, c
             w.ram[Swz<Rl>::f(split_pos(m, I.No, Pr_split))] = v;
         }
         Pr = raman_conv<Rl>(I.resp[ir], I.No, w);
+    }
+    if constexpr (sizeof(Rl) == 8 && !HIL) {
+        if (ip >= 0) {
+            if (M >= 4 * T) plasma_real_f64<4>(I, w, x, M, P, sc, ip, ir, Pr, Pr_split);
+            else if (M >= 2 * T) plasma_real_f64<2>(I, w, x, M, P, sc, ip, ir, Pr, Pr_split);
+            else plasma_real_f64<1>(I, w, x, M, P, sc, ip, ir, Pr, Pr_split);
+            return;
+        }
     }
     PlasmaCarry cr = {0, 0, 0};
     if (ip >= 0) {
