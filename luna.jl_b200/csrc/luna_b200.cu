@@ -646,11 +646,15 @@ int dist_partition(luna_batch* b, const double* pr) {
     b->ndist16 = (int)b->dist16.size();
     b->nreg = (int)b->reg.size();
     const int n16 = std::min(b->ncl16_max, b->ndist16);
-    // a big cluster takes the room of DIST_R_BIG / DIST_R small ones
-    const int ncl = std::min(std::max(1, b->ncl_max - n16 * (DIST_R_BIG / DIST_R)), b->ndist);
+    // a big cluster takes the room of DIST_R_BIG / DIST_R small ones while it runs; the grid of
+    // small clusters is what the device holds without it, so that the ones that find no room
+    // start as soon as big clusters and single CTAs leave their SMs. (A grid cut to the room
+    // left at the start drained the list on 1-5 clusters while the other SMs had run out of work:
+    // 0.27-1.0 s for 96 instances.)
+    const int room = std::min(std::max(1, b->ncl_max - n16 * (DIST_R_BIG / DIST_R)), b->ndist);
     b->dist16_grid = DIST_R_BIG * n16;
-    b->dist_grid = (b->ndist > 0) ? DIST_R * ncl : 0;
-    b->reg_grid = std::max(0, std::min(b->nreg, b->nsm - b->dist_grid - b->dist16_grid));
+    b->dist_grid = DIST_R * std::min(b->ncl_max, b->ndist);
+    b->reg_grid = std::max(0, std::min(b->nreg, b->nsm - DIST_R * room - b->dist16_grid));
     if (b->ndist > 0) CK(cudaMemcpy(b->d_dist, b->dist.data(), sizeof(int) * b->ndist, cudaMemcpyHostToDevice));
     if (b->ndist16 > 0) CK(cudaMemcpy(b->d_dist16, b->dist16.data(), sizeof(int) * b->ndist16, cudaMemcpyHostToDevice));
     if (b->nreg > 0) CK(cudaMemcpy(b->d_reg, b->reg.data(), sizeof(int) * b->nreg, cudaMemcpyHostToDevice));
@@ -750,15 +754,15 @@ int dist_launch(luna_batch* b, const TwTab<Rl>& tw) {
         cfg.numAttrs = 1;
         return cfg;
     };
+    // every kernel is enqueued before the waits that join the streams again: streams share
+    // hardware queues, and a launch behind another stream's wait would start after it
     CK(cudaEventRecord(b->evf, b->stream));
-    if (b->reg_grid > 0) CK(cudaStreamWaitEvent(b->stream2, b->evf, 0));
     if (b->dist16_grid > 0) {
         CK(cudaStreamWaitEvent(b->stream3, b->evf, 0));
         cudaLaunchAttribute at16[1];
         cudaLaunchConfig_t cfg16 = cfg_for(DIST_R_BIG, b->dist16_grid, b->stream3, at16);
         CK(cudaLaunchKernelEx(&cfg16, solve_kernel_dist<Rl, Rl, DIST_R_BIG>, b->d_insts, (const int*)b->d_dist16,
                               b->ndist16, c + 3, (const int*)b->d_reg, b->nreg, c + 1, tw, b->smem));
-        CK(cudaEventRecord(b->evj3, b->stream3));
     }
     if (b->dist_grid > 0) {
         cudaLaunchAttribute at[1];
@@ -766,13 +770,17 @@ int dist_launch(luna_batch* b, const TwTab<Rl>& tw) {
         CK(cudaLaunchKernelEx(&cfg, solve_kernel_dist<Rl, Rl, DIST_R>, b->d_insts, (const int*)b->d_dist, b->ndist, c,
                               (const int*)b->d_reg, b->nreg, c + 1, tw, b->smem));
     }
-    if (b->dist16_grid > 0) CK(cudaStreamWaitEvent(b->stream, b->evj3, 0));
     if (b->reg_grid > 0) {
+        CK(cudaStreamWaitEvent(b->stream2, b->evf, 0));
         solve_kernel<Rl, Rl><<<b->reg_grid, LUNA_BLOCK, b->smem, b->stream2>>>(b->d_insts, b->nreg, c + 1, tw, b->smem,
                                                                               (const int*)b->d_reg);
         CK(cudaEventRecord(b->evj, b->stream2));
-        CK(cudaStreamWaitEvent(b->stream, b->evj, 0));
     }
+    if (b->dist16_grid > 0) {
+        CK(cudaEventRecord(b->evj3, b->stream3));
+        CK(cudaStreamWaitEvent(b->stream, b->evj3, 0));
+    }
+    if (b->reg_grid > 0) CK(cudaStreamWaitEvent(b->stream, b->evj, 0));
     return LUNA_OK;
 }
 
@@ -1340,9 +1348,12 @@ int luna_b200_batch_create(luna_plan* const* plans, int n, const luna_solve_opts
             }
         }
     }
-    if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&b->stream2, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&b->stream3, cudaStreamNonBlocking) != cudaSuccess ||
+    // where SMs come free, the widest clusters are placed first, single CTAs last
+    int plo = 0, phi = 0;
+    cudaDeviceGetStreamPriorityRange(&plo, &phi);
+    if (cudaStreamCreateWithPriority(&b->stream, cudaStreamNonBlocking, std::min(plo, phi + 1)) != cudaSuccess ||
+        cudaStreamCreateWithPriority(&b->stream2, cudaStreamNonBlocking, plo) != cudaSuccess ||
+        cudaStreamCreateWithPriority(&b->stream3, cudaStreamNonBlocking, phi) != cudaSuccess ||
         cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->evf, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->evj, cudaEventDisableTiming) != cudaSuccess ||
