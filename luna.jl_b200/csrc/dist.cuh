@@ -1,6 +1,6 @@
 // Distributed solver: one mode-averaged instance integrated by a thread-block cluster of
 // R CTAs (DIST_R, or DIST_R_BIG for the longest instances), for the long instances of a
-// batch (field-resolved grid, FP64 or mixed precision).
+// batch (FP64; mixed precision on field-resolved grids), and one right-hand side on a cluster.
 //
 // The RK45 loop, stage combinations, error norm and controller are those of
 // solve_instance; what is split is every per-bin and per-sample loop and every transform:
@@ -13,6 +13,8 @@
 //     the bins R k + p, then the blocks are joined by a radix-R step), the forward one
 //     decimation in frequency (radix-R step, then CTA p transforms its sub-sequence), both
 //     on Mb-point Stockham sub-transforms in shared memory;
+//   * envelope grids (FP64): complex transforms of No points on the same scheme, CTA q holding a
+//     contiguous block of complex samples;
 //   * the Raman convolution (a 2M-point transform) on 2R sub-transforms, CTA c holding
 //     the pair {c, 2R - c} ({0, R} for c = 0) so that the real-transform split pairs k with
 //     2M - k inside one CTA.
@@ -33,8 +35,7 @@ namespace luna {
 // elements per thread whose remote loads are issued together
 template <int R>
 struct DUnr {
-    static constexpr int v = 16 / R > 0 ? 16 / R : 1;
-    static constexpr int raman = 8 / R > 0 ? 8 / R : 1;
+    static constexpr int v = R >= 8 ? 16 / R : 2;
 };
 
 namespace dcg = cooperative_groups;
@@ -55,8 +56,11 @@ struct DWs {
     int rank;
 };
 
-__host__ __device__ inline size_t dist_smem_bytes(int No, size_t csize, int R = DIST_R) {
-    const size_t Mb = (size_t)(No / 2) / R;
+// elements of an instance's time-domain buffer: sample pairs (real grids) or complex samples
+__host__ __device__ inline int dist_len(const LunaInst& I) { return I.kind == 0 ? I.No / 2 : I.No; }
+
+__host__ __device__ inline size_t dist_smem_bytes(int len, size_t csize, int R = DIST_R) {
+    const size_t Mb = (size_t)len / R;
     return (csize == 16 ? SmallBytes<double>::v : SmallBytes<float>::v) + 2 * align_up((Mb + 16) * csize, 256) + 4 * align_up(Mb * csize, 256);
 }
 
@@ -69,7 +73,7 @@ __device__ void plan_dws(const LunaInst& I, char* smem, DWs<Rl>& d, const TwTab<
     d.tw = tw;
     d.rank = rank;
     const size_t c = sizeof(cpx<Rl>);
-    const size_t Mb = (size_t)(I.No / 2) / R;
+    const size_t Mb = (size_t)dist_len(I) / R;
     const size_t bs = align_up((Mb + 16) * c, 256), bm = align_up(Mb * c, 256);
     size_t off = SmallBytes<Rl>::v;
     d.stg = reinterpret_cast<cpx<Rl>*>(smem + off);
@@ -98,6 +102,46 @@ __device__ __forceinline__ cpx<Rl> tw_pow(const TwTab<Rl>& tw, unsigned a, int l
     return twiddle<Rl, INV>(tw, (a & ((1u << lg) - 1)) << (TW_LOG_MMAX - lg));
 }
 
+// Join of an inverse transform of R Mb points, transposed: this CTA takes the n1 of its slice
+// [p S, (p + 1) S), S = Mb/R, gathers B_r[n1] from every CTA's fb, forms
+// x[n1 + Mb q] = sum_r W_R^{-r q} B_r[n1] for every q with one in-register DFT and stores each
+// into CTA q's block tb. Each CTA reads Mb values instead of R Mb; the stores are visible after
+// the closing barrier.
+template <typename Rl, int R>
+__device__ __forceinline__ void dist_join(DWs<Rl>& d, int Mb) {
+    const int S = Mb / R, n1b = d.rank * S;
+    for (int j = threadIdx.x; j < S; j += LUNA_BLOCK) {
+        const int pos = Swz<Rl>::f(n1b + j);
+        cpx<Rl> v[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) v[i] = drem(d.fb, bitrev<R>(i))[pos];
+        dft_br<Rl, true, R>(v);
+#pragma unroll
+        for (int q = 0; q < R; ++q) drem(d.tb, q)[pos] = v[q];
+    }
+    dsync();
+}
+
+// Radix-R step of a forward transform of 2^lgM = R Mb points, transposed: this CTA gathers every
+// CTA's block tb at the n1 of its slice, forms y_r = W_M^{r n1} sum_q W_R^{r q} x[n1 + Mb q] for
+// every r with one in-register DFT and stores each into CTA r's sub-transform buffer fb.
+template <typename Rl, int R>
+__device__ __forceinline__ void dist_radix(DWs<Rl>& d, int Mb, int lgM) {
+    const int S = Mb / R, n1b = d.rank * S;
+    for (int j = threadIdx.x; j < S; j += LUNA_BLOCK) {
+        const int n1 = n1b + j;
+        const int pos = Swz<Rl>::f(n1);
+        cpx<Rl> v[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) v[i] = drem(d.tb, bitrev<R>(i))[pos];
+        dft_br<Rl, false, R>(v);
+        drem(d.fb, 0)[pos] = v[0];
+#pragma unroll
+        for (int r = 1; r < R; ++r) drem(d.fb, r)[pos] = v[r] * tw_pow<Rl, false>(d.tw, (unsigned)(r * n1), lgM);
+    }
+    dsync();
+}
+
 // ------------------------------------------------------------------ real transform pair
 // to_time! of a length-2Mc real signal from its spectrum X[n] = load(n), n < Nw (zero up to
 // n = Mc): C2R pre-twiddle Z[n] = (X[n] + conj X[Mc-n]) + i W^-n (X[n] - conj X[Mc-n]) and
@@ -107,7 +151,7 @@ template <typename Rl, int R, typename LoadF>
 __device__ __noinline__ void dist_c2r(DWs<Rl>& d, int Mc, int Nw, LoadF&& load) {
     const int p = d.rank, T = LUNA_BLOCK, tid = threadIdx.x;
     const int Mbc = Mc / R;
-    const int lgM = ilog2i((unsigned)Mc), lgR = ilog2c<R>();
+    const int lgM = ilog2i((unsigned)Mc);
     // DUnr<R>::v own bins per thread and round: their loads are independent and issued together
     for (int j0 = tid; p + R * j0 <= Mc; j0 += DUnr<R>::v * T) {
         cpx<double> X[DUnr<R>::v];
@@ -159,50 +203,7 @@ __device__ __noinline__ void dist_c2r(DWs<Rl>& d, int Mc, int Nw, LoadF&& load) 
         }
     }
     dsync();
-    if constexpr (R == 8 || R == 16) {
-        // join, transposed: this CTA takes the n1 of its slice [p S, (p + 1) S), S = Mbc/R,
-        // gathers B_r[n1] from every CTA, forms x[n1 + Mbc q] = sum_r W_R^{-r q} B_r[n1] for
-        // every q with one in-register DFT and stores each into CTA q's block. Each CTA reads
-        // Mbc values instead of R Mbc; the stores are visible after the closing barrier.
-        const int S = Mbc / R, n1b = p * S;
-        for (int j = tid; j < S; j += T) {
-            const int pos = Swz<Rl>::f(n1b + j);
-            cpx<Rl> v[R];
-#pragma unroll
-            for (int i = 0; i < R; ++i) v[i] = drem(d.fb, bitrev<R>(i))[pos];
-            dft_br<Rl, true, R>(v);
-#pragma unroll
-            for (int q = 0; q < R; ++q) drem(d.tb, q)[pos] = v[q];
-        }
-        dsync();
-    } else {
-    // join: x[n1 + Mbc q] = sum_r W_R^{-r q} B_r[n1], q = this CTA
-    const cpx<Rl>* fr[R];
-    cpx<Rl> wq[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        fr[r] = drem(d.fb, r);
-        wq[r] = tw_pow<Rl, true>(d.tw, (unsigned)(r * p), lgR);
-    }
-    for (int n0 = tid; n0 < Mbc; n0 += DUnr<R>::v * T) {
-        cpx<Rl> v[DUnr<R>::v][R];
-#pragma unroll
-        for (int u = 0; u < DUnr<R>::v; ++u) {
-            const int pos = Swz<Rl>::f(min(n0 + u * T, Mbc - 1));
-#pragma unroll
-            for (int r = 0; r < R; ++r) v[u][r] = fr[r][pos];
-        }
-#pragma unroll
-        for (int u = 0; u < DUnr<R>::v; ++u) {
-            if (n0 + u * T >= Mbc) continue;
-            cpx<Rl> acc = v[u][0];
-#pragma unroll
-            for (int r = 1; r < R; ++r) acc = acc + v[u][r] * wq[r];
-            d.tb[Swz<Rl>::f(n0 + u * T)] = acc;
-        }
-    }
-    __syncthreads();
-    }
+    dist_join<Rl, R>(d, Mbc);
 }
 
 // to_freq! of the sample pairs in tb (every CTA's block): radix-R step, Mbc-point forward
@@ -214,54 +215,9 @@ template <typename Rl, int R, typename StoreF>
 __device__ __noinline__ void dist_r2c(DWs<Rl>& d, int Mc, int Nw, StoreF&& store) {
     const int p = d.rank, T = LUNA_BLOCK, tid = threadIdx.x;
     const int Mbc = Mc / R;
-    const int lgM = ilog2i((unsigned)Mc), lgR = ilog2c<R>();
+    const int lgM = ilog2i((unsigned)Mc);
     dsync();
-    if constexpr (R == 8 || R == 16) {
-        // radix-R step, transposed: this CTA takes the n1 of its slice, gathers every CTA's
-        // block at n1, forms y_r = W_M^{r n1} sum_q W_R^{r q} x[n1 + Mbc q] for every r with
-        // one in-register DFT and stores each into CTA r's sub-transform buffer
-        const int S = Mbc / R, n1b = p * S;
-        for (int j = tid; j < S; j += T) {
-            const int n1 = n1b + j;
-            const int pos = Swz<Rl>::f(n1);
-            cpx<Rl> v[R];
-#pragma unroll
-            for (int i = 0; i < R; ++i) v[i] = drem(d.tb, bitrev<R>(i))[pos];
-            dft_br<Rl, false, R>(v);
-            drem(d.fb, 0)[pos] = v[0];
-#pragma unroll
-            for (int r = 1; r < R; ++r) drem(d.fb, r)[pos] = v[r] * tw_pow<Rl, false>(d.tw, (unsigned)(r * n1), lgM);
-        }
-        dsync();
-    } else {
-    const cpx<Rl>* tr[R];
-    cpx<Rl> wq[R];
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-        tr[q] = drem(d.tb, q);
-        wq[q] = tw_pow<Rl, false>(d.tw, (unsigned)(p * q), lgR);
-    }
-    for (int n0 = tid; n0 < Mbc; n0 += DUnr<R>::v * T) {
-        cpx<Rl> v[DUnr<R>::v][R];
-#pragma unroll
-        for (int u = 0; u < DUnr<R>::v; ++u) {
-            const int pos = Swz<Rl>::f(min(n0 + u * T, Mbc - 1));
-#pragma unroll
-            for (int q = 0; q < R; ++q) v[u][q] = tr[q][pos];
-        }
-#pragma unroll
-        for (int u = 0; u < DUnr<R>::v; ++u) {
-            const int n1 = n0 + u * T;
-            if (n1 >= Mbc) continue;
-            cpx<Rl> acc = v[u][0];
-#pragma unroll
-            for (int q = 1; q < R; ++q) acc = acc + v[u][q] * wq[q];
-            if (p) acc = acc * tw_pow<Rl, false>(d.tw, (unsigned)(p * n1), lgM);
-            d.fb[Swz<Rl>::f(n1)] = acc;
-        }
-    }
-    __syncthreads();
-    }
+    dist_radix<Rl, R>(d, Mbc, lgM);
     fft_sub1<Rl, false>(d.fb, Mbc, d.tw);
     dsync();
     const int po = (R - p) % R;
@@ -293,20 +249,49 @@ __device__ __noinline__ void dist_r2c(DWs<Rl>& d, int Mc, int Nw, StoreF&& store
     __syncthreads();
 }
 
+// ------------------------------------------------------------------ complex transform pair
+// Envelope grids (FP64): inverse transform of the M bins X[n] = load(n) into this CTA's block of
+// samples tb (unscaled), and back; the steps of the real pair without its split.
+template <int R, typename LoadF>
+__device__ __noinline__ void dist_c2c_inv(DWs<double>& d, int M, LoadF&& load) {
+    const int p = d.rank, Mb = M / R, lgM = ilog2i((unsigned)M);
+    for (int k = threadIdx.x; k < Mb; k += LUNA_BLOCK) d.fb[Swz<double>::f(k)] = load(R * k + p);
+    __syncthreads();
+    fft_sub1<double, true>(d.fb, Mb, d.tw);
+    if (p)
+        for (int n1 = threadIdx.x; n1 < Mb; n1 += LUNA_BLOCK) {
+            const int pos = Swz<double>::f(n1);
+            d.fb[pos] = d.fb[pos] * tw_pow<double, true>(d.tw, (unsigned)(p * n1), lgM);
+        }
+    dsync();
+    dist_join<double, R>(d, Mb);
+}
+// store(n, X[n]) for the own bins n = p (mod R)
+template <int R, typename StoreF>
+__device__ __noinline__ void dist_c2c_fwd(DWs<double>& d, int M, StoreF&& store) {
+    const int Mb = M / R;
+    dsync();
+    dist_radix<double, R>(d, Mb, ilog2i((unsigned)M));
+    fft_sub1<double, false>(d.fb, Mb, d.tw);
+    for (int k = threadIdx.x; k < Mb; k += LUNA_BLOCK) store(R * k + d.rank, d.fb[Swz<double>::f(k)]);
+    __syncthreads();
+}
+
 // ------------------------------------------------------------------ Raman convolution
-// The 2M-point transform of z[m] = (E[2m]^2, E[2m+1]^2) (m < M, zero above) on 2R
-// sub-transforms of Mb points, its real-transform split, the response product and the
+// The 2M-point transform of z[m] = (E[2m]^2, E[2m+1]^2) (m < M, zero above; SQ: from the field
+// pairs in src, else z itself is in src) on 2R sub-transforms of Mb points, its real-transform split, the response product and the
 // inverse split (as raman_conv), then the inverse sub-transforms; rb0/rb1 end holding
 // B_p[n1] = W_2M^{-p n1} IFFT_Mb(Y_p)[n1] for this CTA's pair of sub-transforms. Needs
 // every CTA's field block (call after a cluster barrier).
-template <typename Rl, int R>
-__device__ __noinline__ void dist_raman_fwd(const LunaResp& rr, DWs<Rl>& d, int M, double sc) {
+template <typename Rl, int R, bool SQ>
+__device__ __noinline__ void dist_raman_fwd(const LunaResp& rr, DWs<Rl>& d, cpx<Rl>* src, int M, double sc) {
     const int c = d.rank, T = LUNA_BLOCK, tid = threadIdx.x;
     const int Mb = M / R, Mr = 2 * M;
-    const int lgMr = ilog2i((unsigned)Mr), lg2R = ilog2c<R>() + 1;
+    const int lgMr = ilog2i((unsigned)Mr);
+    [[maybe_unused]] const int lg2R = ilog2c<R>() + 1;
     const int pa = (c == 0) ? 0 : c, pb = (c == 0) ? R : 2 * R - c;
     const Rl s = (Rl)sc;
-    if constexpr (R == 8) {
+    if constexpr (R <= 8) {
         // the radix-2R step, transposed: this CTA takes the n1 of its slice, squares every
         // CTA's field pair at n1, forms X_f = sum_q W_2R^{f q} z[n1 + Mb q] for all 2R
         // sub-transforms f with one in-register DFT (z is zero for q >= R) and stores
@@ -322,9 +307,13 @@ __device__ __noinline__ void dist_raman_fwd(const LunaResp& rr, DWs<Rl>& d, int 
             for (int i = 0; i < R2; ++i) {
                 const int q = bitrev<R2>(i);
                 if (q < R) {
-                    const cpx<Rl> e = drem(d.tb, q)[pos];
-                    const Rl e0 = e.x * s, e1 = e.y * s;
-                    v[i] = mk<Rl>(e0 * e0, e1 * e1);
+                    const cpx<Rl> e = drem(src, q)[pos];
+                    if constexpr (SQ) {
+                        const Rl e0 = e.x * s, e1 = e.y * s;
+                        v[i] = mk<Rl>(e0 * e0, e1 * e1);
+                    } else {
+                        v[i] = e;
+                    }
                 } else {
                     v[i] = mk<Rl>(0, 0);
                 }
@@ -339,7 +328,8 @@ __device__ __noinline__ void dist_raman_fwd(const LunaResp& rr, DWs<Rl>& d, int 
             }
         }
         dsync();
-    } else if constexpr (R == 16) {
+    } else {
+        static_assert(R == 16, "cluster sizes: 4, 8, 16");
         // the same transposed step with the 2R-point DFT as two R-point ones (a 2R-point
         // one does not fit in registers): z is zero for q >= R, so
         // X_{2g+e} = sum_{q<R} W_R^{g q} (W_2R^{e q} z_q), e = 0, 1; each half gathers the
@@ -354,9 +344,13 @@ __device__ __noinline__ void dist_raman_fwd(const LunaResp& rr, DWs<Rl>& d, int 
 #pragma unroll
                 for (int i = 0; i < R; ++i) {
                     const int q = bitrev<R>(i);
-                    const cpx<Rl> ev = drem(d.tb, q)[pos];
-                    const Rl e0 = ev.x * s, e1 = ev.y * s;
-                    v[i] = mk<Rl>(e0 * e0, e1 * e1);
+                    const cpx<Rl> ev = drem(src, q)[pos];
+                    if constexpr (SQ) {
+                        const Rl e0 = ev.x * s, e1 = ev.y * s;
+                        v[i] = mk<Rl>(e0 * e0, e1 * e1);
+                    } else {
+                        v[i] = ev;
+                    }
                     if (e && q) v[i] = v[i] * tw_pow<Rl, false>(d.tw, (unsigned)q, lg2R);
                 }
                 dft_br<Rl, false, R>(v);
@@ -370,48 +364,6 @@ __device__ __noinline__ void dist_raman_fwd(const LunaResp& rr, DWs<Rl>& d, int 
             }
         }
         dsync();
-    } else {
-    const cpx<Rl>* tr[R];
-    cpx<Rl> wa[R], wb[R];
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-        tr[q] = drem(d.tb, q);
-        wa[q] = tw_pow<Rl, false>(d.tw, (unsigned)(pa * q), lg2R);
-        wb[q] = tw_pow<Rl, false>(d.tw, (unsigned)(pb * q), lg2R);
-    }
-    for (int n0 = tid; n0 < Mb; n0 += DUnr<R>::v * T) {
-      cpx<Rl> ev[DUnr<R>::v][R];
-#pragma unroll
-      for (int u = 0; u < DUnr<R>::v; ++u) {
-          const int pos = Swz<Rl>::f(min(n0 + u * T, Mb - 1));
-#pragma unroll
-          for (int q = 0; q < R; ++q) ev[u][q] = tr[q][pos];
-      }
-#pragma unroll
-      for (int u = 0; u < DUnr<R>::v; ++u) {
-        const int n1 = n0 + u * T;
-        if (n1 >= Mb) continue;
-        const int pos = Swz<Rl>::f(n1);
-        cpx<Rl> z[R];
-#pragma unroll
-        for (int q = 0; q < R; ++q) {
-            const cpx<Rl> e = ev[u][q];
-            const Rl e0 = e.x * s, e1 = e.y * s;
-            z[q] = mk<Rl>(e0 * e0, e1 * e1);
-        }
-        cpx<Rl> a = z[0], b = z[0];
-#pragma unroll
-        for (int q = 1; q < R; ++q) {
-            a = a + z[q] * wa[q];
-            b = b + z[q] * wb[q];
-        }
-        if (pa) a = a * tw_pow<Rl, false>(d.tw, (unsigned)(pa * n1), lgMr);
-        b = b * tw_pow<Rl, false>(d.tw, (unsigned)(pb * n1), lgMr);
-        d.rb0[pos] = a;
-        d.rb1[pos] = b;
-      }
-    }
-    __syncthreads();
     }
     fft_sub2<Rl, false>(d.rb0, d.rb1, Mb, d.tw);
     // pairs (f, Mr - f) with f = 2R k + p; Zk/Zm are entries of the complex transform
@@ -460,65 +412,8 @@ __device__ __noinline__ void dist_raman_fwd(const LunaResp& rr, DWs<Rl>& d, int 
     __syncthreads();
 }
 
-// Raman polarisation pair of this CTA's block at n1 from every CTA's B_p (after a barrier
-// that follows dist_raman_fwd in every CTA): P[n1 + Mb q] = sum_p W_2R^{-p q} B_p[n1].
-template <typename Rl, int R>
-struct RamanOut {
-    const cpx<Rl>* b0[R];
-    const cpx<Rl>* b1[R];
-    cpx<Rl> w0[R], w1[R];
-    __device__ void init(DWs<Rl>& d) {
-        const int q = d.rank, lg2R = ilog2c<R>() + 1;
-#pragma unroll
-        for (int c = 0; c < R; ++c) {
-            b0[c] = drem(d.rb0, c);
-            b1[c] = drem(d.rb1, c);
-            const int pa = (c == 0) ? 0 : c, pb = (c == 0) ? R : 2 * R - c;
-            w0[c] = tw_pow<Rl, true>(d.tw, (unsigned)(pa * q), lg2R);
-            w1[c] = tw_pow<Rl, true>(d.tw, (unsigned)(pb * q), lg2R);
-        }
-    }
-    // P for the pairs n1 = tid + k T of this CTA's block into out[Swz(n1)] (remote loads of
-    // two pairs in flight together)
-    __device__ void block(cpx<Rl>* out, int Mb) const {
-        constexpr int U = DUnr<R>::raman;
-        for (int n0 = threadIdx.x; n0 < Mb; n0 += U * LUNA_BLOCK) {
-            cpx<Rl> v0[U][R], v1[U][R];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int pos = Swz<Rl>::f(min(n0 + u * LUNA_BLOCK, Mb - 1));
-#pragma unroll
-                for (int c = 0; c < R; ++c) {
-                    v0[u][c] = b0[c][pos];
-                    v1[u][c] = b1[c][pos];
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int n1 = n0 + u * LUNA_BLOCK;
-                if (n1 >= Mb) continue;
-                cpx<Rl> acc = v0[u][0] + v1[u][0] * w1[0];
-#pragma unroll
-                for (int c = 1; c < R; ++c) acc = acc + v0[u][c] * w0[c] + v1[u][c] * w1[c];
-                out[Swz<Rl>::f(n1)] = acc;
-            }
-        }
-    }
-    __device__ __forceinline__ cpx<Rl> at(int pos) const {
-        cpx<Rl> v0[R], v1[R];
-#pragma unroll
-        for (int c = 0; c < R; ++c) {
-            v0[c] = b0[c][pos];
-            v1[c] = b1[c][pos];
-        }
-        cpx<Rl> acc = v0[0] + v1[0] * w1[0];
-#pragma unroll
-        for (int c = 1; c < R; ++c) acc = acc + v0[c] * w0[c] + v1[c] * w1[c];
-        return acc;
-    }
-};
-
-// RamanOut::block transposed for clusters of 8 and 16: this CTA takes the n1 of its slice
+// Raman polarisation P[n1 + Mb q] = sum_p W_2R^{-p q} B_p[n1] of every block, transposed (after a
+// barrier that follows dist_raman_fwd in every CTA): this CTA takes the n1 of its slice
 // [r S, (r + 1) S), S = Mb/R, gathers the 2R sub-transform values B_p[n1] (two per CTA),
 // forms P[n1 + Mb q] = sum_p W_2R^{-p q} B_p[n1] for every q with one in-register DFT and
 // stores each into CTA q's out. Each CTA reads 2 Mb values instead of 2 R Mb; the stores
@@ -676,13 +571,7 @@ __device__ __noinline__ void dist_plasma(const LunaInst& I, DWs<Rl>& d, int M, d
     if (ir >= 0) {
         // the Raman polarisation of this block into tb (the field now lives in ev); with the
         // transposed form other CTAs write it, visible after the next barriers below
-        if constexpr (R == 8 || R == 16) {
-            raman_out_scatter<Rl, R>(d, d.tb, Mb);
-        } else {
-            RamanOut<Rl, R> ro;
-            ro.init(d);
-            ro.block(d.tb, Mb);
-        }
+        raman_out_scatter<Rl, R>(d, d.tb, Mb);
     }
     double c1 = 0;
     for (int j = 0; j < q; ++j) c1 += drem(d.xs, j)[0];
@@ -915,19 +804,12 @@ __device__ __noinline__ void dist_pointwise(const LunaInst& I, DWs<Rl>& d, int M
         return;
     }
     dsync();  // every field block complete; every read of the sub-transforms done
-    if (ir >= 0) dist_raman_fwd<Rl, R>(I.resp[ir], d, M, sc);
+    if (ir >= 0) dist_raman_fwd<Rl, R, true>(I.resp[ir], d, d.tb, M, sc);
     if (ip < 0) {
         dsync();  // every CTA's Raman sub-transforms ready; every read of the field blocks done
         // the sub-transform buffer is free after the barrier above
-        if constexpr (R == 8 || R == 16) {
-            raman_out_scatter<Rl, R>(d, d.fb, Mb);
-            dsync();  // every CTA's stores into this block
-        } else {
-            RamanOut<Rl, R> ro;
-            ro.init(d);
-            ro.block(d.fb, Mb);
-            __syncthreads();
-        }
+        raman_out_scatter<Rl, R>(d, d.fb, Mb);
+        dsync();  // every CTA's stores into this block
         for (int n1 = tid; n1 < Mb; n1 += T) {
             const int pos = Swz<Rl>::f(n1);
             const cpx<Rl> e = d.tb[pos];
@@ -948,12 +830,78 @@ __device__ __noinline__ void dist_pointwise(const LunaInst& I, DWs<Rl>& d, int M
             case 8: dist_plasma_f64<8, R>(I, d, M, sc, ip, ir, kc, rc); break;
             default: dist_plasma_f64<16, R>(I, d, M, sc, ip, ir, kc, rc); break;
         }
-    } else
+    } else {
     switch (2 * Mb / T) {
         case 4: dist_plasma<Rl, 4, R>(I, d, M, sc, ip, ir, kc, rc); break;
         case 8: dist_plasma<Rl, 8, R>(I, d, M, sc, ip, ir, kc, rc); break;
         default: dist_plasma<Rl, 16, R>(I, d, M, sc, ip, ir, kc, rc); break;
     }
+    }
+}
+
+// Envelope grids (FP64): Kerr_env, Kerr_env_thg and RamanPolarEnv (pointwise_env) on this CTA's
+// block of samples tb, in place; the squares of the Raman convolution go as pairs of consecutive
+// samples through the real grids' transforms (M = No/2 pairs).
+template <int R>
+__device__ __noinline__ void dist_pointwise_env(const LunaInst& I, DWs<double>& d, double sc) {
+    const int T = LUNA_BLOCK, tid = threadIdx.x;
+    const int Mb = I.No / R, n0 = d.rank * Mb;
+    int ir = -1;
+    for (int i = 0; i < I.nresp; ++i)
+        if (I.resp[i].kind == LUNA_RESP_RAMAN) ir = i;
+    if (ir >= 0) {
+        for (int m = tid; m < Mb / 2; m += T) {
+            const cpx<double> a = scale(sc, d.tb[Swz<double>::f(2 * m)]), b = scale(sc, d.tb[Swz<double>::f(2 * m + 1)]);
+            d.stg[Swz<double>::f(m)] = mk<double>(0.5 * abs2(a), 0.5 * abs2(b));
+        }
+        dsync();
+        dist_raman_fwd<double, R, false>(I.resp[ir], d, d.stg, I.No / 2, 1.0);
+        dsync();  // every CTA's sub-transforms ready
+        raman_out_scatter<double, R>(d, d.fb, Mb / 2);
+        dsync();  // every CTA's stores into this block
+    }
+    for (int n1 = tid; n1 < Mb; n1 += T) {
+        const int pos = Swz<double>::f(n1);
+        const cpx<double> E = scale(sc, d.tb[pos]);
+        cpx<double> Pt = mk<double>(0, 0);
+        for (int i = 0; i < I.nresp; ++i) {
+            const LunaResp& r = I.resp[i];
+            if (r.kind == LUNA_RESP_KERR_ENV && r.cthg) {
+                const cpx<double> C = ldg(reinterpret_cast<const cpx<double>*>(r.cthg) + n0 + n1);
+                Pt = Pt + scale(0.25 * r.coef, scale(3.0 * abs2(E), E) + C * (E * E) * E);
+            } else if (r.kind == LUNA_RESP_KERR_ENV) {
+                Pt = Pt + scale(0.75 * r.coef * abs2(E), E);
+            } else if (i == ir) {
+                const cpx<double> p = d.fb[Swz<double>::f(n1 >> 1)];
+                Pt = Pt + scale(r.coef * ((n1 & 1) ? p.y : p.x), E);
+            }
+        }
+        d.tb[pos] = scale(__ldg(I.towin + n0 + n1), Pt);
+    }
+    __syncthreads();
+}
+
+// One right-hand side on a cluster: bin i of the stage input from load(i), store(i, v) takes bin i
+// of the output (own bins of this CTA).
+template <typename Rl, int R, typename LoadF, typename StoreF>
+__device__ __forceinline__ void dist_rhs(const LunaInst& I, DWs<Rl>& d, LoadF&& load, StoreF&& store) {
+    const cpx<double>* of = reinterpret_cast<const cpx<double>*>(I.outfac);
+    if constexpr (sizeof(Rl) == 8) {
+        if (I.kind == 1) {
+            // copy_scale_both! padding and cropping (env_to_time, env_to_freq)
+            const int No = I.No, N = I.N, h = I.N / 2;
+            dist_c2c_inv<R>(d, No, [&](int j) { return j < h ? load(j) : j >= No - h ? load(j - No + N) : mk<double>(0, 0); });
+            dist_pointwise_env<R>(I, d, I.in_scale);
+            dist_c2c_fwd<R>(d, No, [&](int j, cpx<double> X) {
+                const int k = j < h ? j : j - No + N;
+                if (j < h || j >= No - h) store(k, X * ldg(of + k));
+            });
+            return;
+        }
+    }
+    dist_c2r<Rl, R>(d, I.No / 2, I.Nw, load);
+    dist_pointwise<Rl, R>(I, d, I.No / 2, I.in_scale);
+    dist_r2c<Rl, R>(d, I.No / 2, I.Nw, [&](int kb, cpx<double> X) { store(kb, X * ldg(of + kb)); });
 }
 
 // ------------------------------------------------------------------ the integrator
@@ -961,10 +909,9 @@ __device__ __noinline__ void dist_pointwise(const LunaInst& I, DWs<Rl>& d, int M
 template <typename Rl, typename Kt, int R>
 __device__ __noinline__ void solve_instance_dist(LunaInst& I, DWs<Rl>& d, Ctl& c) {
     const int p = d.rank, T = LUNA_BLOCK, tid = threadIdx.x;
-    const int Nw = I.Nw, M = I.No / 2, Mcoarse = I.N / 2;
+    const int Nw = I.Nw, Mcoarse = I.N / 2;
     const bool writer = (p == 0);
     const cpx<double>* L = reinterpret_cast<const cpx<double>*>(I.linop);
-    const cpx<double>* of = reinterpret_cast<const cpx<double>*>(I.outfac);
     void** k = c.k;
     if (tid == 0) {
         for (int j = 0; j < 7; ++j) k[j] = I.k[j];
@@ -995,12 +942,7 @@ __device__ __noinline__ void solve_instance_dist(LunaInst& I, DWs<Rl>& d, Ctl& c
         }
     }
     __syncthreads();
-    const double sc = I.in_scale;
-    auto rhs_d = [&](auto&& load, auto&& store) {
-        dist_c2r<Rl, R>(d, M, Nw, load);
-        dist_pointwise<Rl, R>(I, d, M, sc);
-        dist_r2c<Rl, R>(d, M, Nw, [&](int kb, cpx<double> X) { store(kb, X * ldg(of + kb)); });
-    };
+    auto rhs_d = [&](auto&& load, auto&& store) { dist_rhs<Rl, R>(I, d, load, store); };
     {
         const cpx<double>* y = reinterpret_cast<const cpx<double>*>(py);
         void* k0 = k[0];
@@ -1134,9 +1076,23 @@ __device__ __noinline__ void solve_instance_dist(LunaInst& I, DWs<Rl>& d, Ctl& c
             {
                 cpx<double>* Yo = reinterpret_cast<cpx<double>*>(pyn);
                 const double inv = 1.0 / (double)I.N;
-                dist_c2r<Rl, R>(d, Mcoarse, Nw, [&](int i) -> cpx<double> {
-                    return scale(__ldg(I.wwin + i), Yo[i] * e1[i]);
-                });
+                auto win = [&](int i) -> cpx<double> { return scale(__ldg(I.wwin + i), Yo[i] * e1[i]); };
+                bool env = false;
+                if constexpr (sizeof(Rl) == 8) {
+                    env = I.kind == 1;
+                    if (env) {
+                        const int Mb = I.N / R;
+                        dist_c2c_inv<R>(d, I.N, win);
+                        for (int n1 = tid; n1 < Mb; n1 += T) {
+                            const int pos = Swz<double>::f(n1);
+                            d.tb[pos] = scale(inv * __ldg(I.twin + p * Mb + n1), d.tb[pos]);
+                        }
+                        __syncthreads();
+                        dist_c2c_fwd<R>(d, I.N, [&](int i, cpx<double> X) { Yo[i] = X; });
+                    }
+                }
+                if (!env) {
+                dist_c2r<Rl, R>(d, Mcoarse, Nw, win);
                 const int Mbc = Mcoarse / R;
                 for (int n1 = tid; n1 < Mbc; n1 += T) {
                     const int pos = Swz<Rl>::f(n1);
@@ -1148,6 +1104,7 @@ __device__ __noinline__ void solve_instance_dist(LunaInst& I, DWs<Rl>& d, Ctl& c
                 }
                 __syncthreads();
                 dist_r2c<Rl, R>(d, Mcoarse, Nw, [&](int i, cpx<double> X) { Yo[i] = X; });
+                }
             }
             while (saved < I.saveN && I.zsave[saved] <= c.tn) {
                 interpolate_row<Rl, Kt>(Nw, I.linop, c, I.zsave[saved], k, py, pyn,

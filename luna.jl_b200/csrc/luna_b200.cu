@@ -385,6 +385,31 @@ rhs_kernel(LunaInst* inst, const double2* Ew, double2* nl, TwTab<Rl> tw, int sme
     if (threadIdx.x == 0) *status = (*w.flag & (1 << ST_FIELD_ABOVE_EMAX)) ? ST_FIELD_ABOVE_EMAX : ST_OK;
 }
 
+// The same on a cluster of R CTAs in FP64 (constant fill, no analytic-signal responses), the
+// right-hand side of the distributed solver. Bound by latency as on one CTA, but every loop over
+// bins and samples is 1/R as long and the sub-transforms are log2 R levels shorter.
+template <int R>
+__global__ void __launch_bounds__(LUNA_BLOCK, 1)
+rhs_kernel_dist(const LunaInst* inst, const double2* Ew, double2* nl, TwTab<double> tw, int* status) {
+    __shared__ LunaInst sI;
+    tws_fill(tw);
+    const LunaInst& I = local_inst<double>(inst, &sI);
+    DWs<double> d;
+    plan_dws<double, R>(I, dsm, d, tw, (int)cooperative_groups::this_cluster().block_rank());
+    if (threadIdx.x == 0) *d.flag = 0;
+    dsync();  // every CTA of the cluster has started before its shared memory is addressed
+    const cpx<double>* E = reinterpret_cast<const cpx<double>*>(Ew);
+    cpx<double>* o = reinterpret_cast<cpx<double>*>(nl);
+    dist_rhs<double, R>(I, d, [&](int k) { return E[k]; }, [&](int k, cpx<double> v) { o[k] = v; });
+    dsync();
+    if (d.rank == 0 && threadIdx.x == 0) {
+        int fl = 0;
+        for (int j = 0; j < R; ++j) fl |= *drem(d.flag, j);
+        *status = (fl & (1 << ST_FIELD_ABOVE_EMAX)) ? ST_FIELD_ABOVE_EMAX : ST_OK;
+    }
+    dsync();  // rank 0 has read the others' flags
+}
+
 // linop!(out, z) of a pressure-gradient plan and the output factor at z, on one CTA.
 __global__ void __launch_bounds__(LUNA_BLOCK, 1)
 grad_linop_kernel(LunaInst I, double z, double2* L, double2* of) {
@@ -543,6 +568,7 @@ struct luna_plan {
     double2* d_nl = nullptr;
     int* d_status = nullptr;
     cudaStream_t stream = nullptr;
+    int rhs_R = 0;               // CTAs of a right-hand side (0: not decided yet)
 };
 
 struct luna_batch {
@@ -612,27 +638,95 @@ void free_all(std::vector<void*>& allocs) {
     allocs.clear();
 }
 
-// Which instances of a batch run distributed, from per-instance work estimates: the eligible
-// ones whose estimate is at least the mean load of an SM (total / SMs), i.e. the long poles
-// of the batch (a cluster costs more SM time than one CTA; shorter Raman instances whose
-// buffers overflow one CTA run single with them in global memory). Every SM that can hold a
-// cluster starts as one (longest instances first); the single-CTA instances fill the SMs
-// left over and the clusters once their list is empty. Both lists in priority order.
+// Clusters of R CTAs of `kern` (sm bytes of dynamic shared memory) that fit on the device at once;
+// raises the kernel's limits (to the device's, so that callers of different sizes never lower each
+// other's).
+template <typename K>
+int max_clusters(K kern, int R, int sm) {
+    int ncl = 0;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = R;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(R * 32, 1, 1);
+    cfg.blockDim = dim3(LUNA_BLOCK, 1, 1);
+    cfg.dynamicSmemBytes = sm;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin()) != cudaSuccess ||
+        (R > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
+        cudaOccupancyMaxActiveClusters(&ncl, kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return ncl;
+}
+
+// Whether an instance can run on a cluster of R CTAs: at least two samples a thread in FP64 (four
+// in mixed precision) and sub-transforms that one CTA holds.
+template <typename Rl>
+bool dist_fits(const LunaInst& I, int R) {
+    const int len = dist_len(I), Mc = I.kind == 0 ? I.N / 2 : I.N;
+    if (I.grad || needs_hilbert(I) || (I.kind == 1 && sizeof(Rl) == 4)) return false;
+    const int least = (sizeof(Rl) == 8 ? 1 : 2) * LUNA_BLOCK;
+    return len % R == 0 && len / R >= least && len / R <= FftEmax<Rl>::v * LUNA_BLOCK && Mc % R == 0 && Mc / R >= 64 &&
+           Mc <= len && I.Nw <= Mc + 1 && dist_smem_bytes(len, sizeof(cpx<Rl>), R) <= (size_t)max_smem_optin();
+}
+
+// Which instances of a batch run distributed, from per-instance work estimates (single-CTA time in
+// any unit). Mixed precision: the eligible ones whose estimate is at least the mean load of an SM
+// (total / SMs), i.e. the long poles of the batch, on clusters of DIST_R, from four times that on
+// DIST_R_BIG. FP64: the number k of instances, longest first, for which the larger of the mean
+// SM load and the longest single run is smallest, a cluster of DIST_R taking 1/3 of the time of one CTA
+// (measured 2.5-4) and so 8/3 of its SM time; all of them on DIST_R_BIG when that many fit at
+// once (a cluster of 16 takes about 3/4 of the time of one of 8, i.e. more SM time). Shapes set
+// per instance come first. Every SM that can hold a cluster starts as one (longest instances
+// first); the single-CTA instances fill the SMs left over and the clusters once their list is
+// empty. All lists in priority order.
 int dist_partition(luna_batch* b, const double* pr) {
     const int n = b->n;
+    // 0: one CTA, 1: a cluster of DIST_R, 2: a cluster of DIST_R_BIG
+    std::vector<char> isd(n, 0), big(n, 0);
+    for (int i : b->elig16) big[i] = b->ncl16_max > 0;
+    auto shape = [&](int i) { return b->shape.empty() ? 0 : b->shape[i]; };
     double W = 0;
     for (int i = 0; i < n; ++i) W += pr[i];
-    const double thr = W / std::max(1, b->nsm);
-    // 0: one CTA, 1: a cluster of DIST_R, 2: a cluster of DIST_R_BIG. The big clusters take
-    // the eligible instances whose estimate is at least four times the mean SM load (those
-    // that would set the makespan even on a cluster of DIST_R)
-    std::vector<char> isd(n, 0), big(n, 0);
-    for (int i = 0; i < n; ++i) big[i] = 0;
-    for (int i : b->elig16) big[i] = 1;
-    for (int i : b->elig) {
-        const int sh = b->shape.empty() ? 0 : b->shape[i];
-        isd[i] = sh == 2 || sh == 3 || (sh == 0 && pr[i] >= thr);
-        if (isd[i] && big[i] && b->ncl16_max > 0 && (sh == 3 || (sh == 0 && pr[i] >= 4.0 * thr))) isd[i] = 2;
+    if (b->precision == LUNA_PREC_FP64) {
+        std::vector<int> ord(b->elig);
+        std::stable_sort(ord.begin(), ord.end(), [&](int a, int c) { return pr[a] > pr[c]; });
+        std::vector<char> el(n, 0);
+        for (int i : ord) el[i] = 1;
+        double rest = 0;  // longest instance that cannot be distributed
+        for (int i = 0; i < n; ++i)
+            if (!el[i]) rest = std::max(rest, pr[i]);
+        double best = 0, load = W;
+        size_t k = 0;
+        for (size_t j = 0; j <= ord.size(); ++j) {
+            if (j > 0) load += (8.0 / 3.0 - 1.0) * pr[ord[j - 1]];
+            const double longest = std::max(std::max(rest, j < ord.size() ? pr[ord[j]] : 0.0), j > 0 ? pr[ord[0]] / 3.0 : 0.0);
+            const double t = std::max(load / std::max(1, b->nsm), longest);
+            if (j == 0 || t < best) {
+                best = t;
+                k = j;
+            }
+        }
+        for (size_t j = 0; j < k; ++j)
+            if (shape(ord[j]) == 0) isd[ord[j]] = 1;
+        for (int i : ord)
+            if (shape(i) >= 2) isd[i] = 1;
+        int nd = 0;
+        for (int i = 0; i < n; ++i) nd += isd[i];
+        for (int i = 0; i < n; ++i)
+            if (isd[i] && big[i] && (shape(i) == 3 || (shape(i) == 0 && nd <= b->ncl16_max))) isd[i] = 2;
+    } else {
+        const double thr = W / std::max(1, b->nsm);
+        for (int i : b->elig) {
+            const int sh = shape(i);
+            isd[i] = sh == 2 || sh == 3 || (sh == 0 && pr[i] >= thr);
+            if (isd[i] && big[i] && (sh == 3 || (sh == 0 && pr[i] >= 4.0 * thr))) isd[i] = 2;
+        }
     }
     b->dist.clear();
     b->dist16.clear();
@@ -668,60 +762,26 @@ int dist_partition(luna_batch* b, const double* pr) {
 template <typename Rl>
 int dist_setup(luna_batch* b, const luna_solve_opts* opts, int nsm) {
     const int n = b->n;
-    const int maxs = max_smem_optin();
-    const size_t cs = sizeof(cpx<Rl>);
     std::vector<int> dl, dl16;
     std::vector<double> cost(n);
-    size_t dsm = 0;
-    const int dmin = opts->dist_min_no > 0 ? opts->dist_min_no : 16384;
-    auto fits = [&](const LunaInst& I, int R) {
-        const int M = I.No / 2, Mc = I.N / 2;
-        return M % R == 0 && M / R >= 2 * LUNA_BLOCK && M / R <= FftEmax<Rl>::v * LUNA_BLOCK && Mc % R == 0 &&
-               Mc / R >= 64 && Mc <= M && I.Nw <= Mc + 1 && dist_smem_bytes(I.No, cs, R) <= (size_t)maxs;
-    };
+    size_t dsm_b = 0;
+    const int dmin = opts->dist_min_no > 0 ? opts->dist_min_no : (sizeof(Rl) == 8 ? 4096 : 16384);
     for (int i = 0; i < n; ++i) {
         const LunaInst& I = b->h[i];
-        const bool ok = I.kind == 0 && !I.grad && !needs_hilbert(I) && opts->stats_cap <= 0 && I.No >= dmin &&
-                        fits(I, DIST_R);
-        if (ok) {
+        if (opts->stats_cap <= 0 && I.No >= dmin && dist_fits<Rl>(I, DIST_R)) {
             dl.push_back(i);
-            dsm = std::max(dsm, dist_smem_bytes(I.No, cs));
-            if (fits(I, DIST_R_BIG)) dl16.push_back(i);
+            dsm_b = std::max(dsm_b, dist_smem_bytes(dist_len(I), sizeof(cpx<Rl>)));
+            if (dist_fits<Rl>(I, DIST_R_BIG)) dl16.push_back(i);
         }
         cost[i] = (double)I.No * std::log2((double)I.No) * (has_raman(I) ? 2.0 : 1.0);
     }
     if (dl.empty()) return LUNA_OK;
-    const int sm = (int)std::max<size_t>((size_t)b->smem, dsm);
-    if (cudaFuncSetAttribute(solve_kernel_dist<Rl, Rl, DIST_R>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) != cudaSuccess ||
-        cudaFuncSetAttribute(solve_kernel<Rl, Rl>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) != cudaSuccess)
+    const int sm = (int)std::max<size_t>((size_t)b->smem, dsm_b);
+    if (cudaFuncSetAttribute(solve_kernel<Rl, Rl>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) != cudaSuccess)
         return fail(LUNA_ERR_CUDA, "batch_create: cannot set shared memory size (distributed solver)");
-    auto max_clusters = [&](auto kern, int R) {
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = R;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.gridDim = dim3(R * 32, 1, 1);
-        cfg.blockDim = dim3(LUNA_BLOCK, 1, 1);
-        cfg.dynamicSmemBytes = sm;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        int ncl = 0;
-        if (cudaOccupancyMaxActiveClusters(&ncl, kern, &cfg) != cudaSuccess) {
-            cudaGetLastError();
-            ncl = 0;
-        }
-        return ncl;
-    };
-    const int ncl = max_clusters(solve_kernel_dist<Rl, Rl, DIST_R>, DIST_R);
+    const int ncl = max_clusters(solve_kernel_dist<Rl, Rl, DIST_R>, DIST_R, sm);
     if (ncl < 1) return LUNA_OK;
-    int ncl16 = 0;
-    if (!dl16.empty() &&
-        cudaFuncSetAttribute(solve_kernel_dist<Rl, Rl, DIST_R_BIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) == cudaSuccess &&
-        cudaFuncSetAttribute(solve_kernel_dist<Rl, Rl, DIST_R_BIG>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)
-        ncl16 = max_clusters(solve_kernel_dist<Rl, Rl, DIST_R_BIG>, DIST_R_BIG);
-    cudaGetLastError();
+    const int ncl16 = dl16.empty() ? 0 : max_clusters(solve_kernel_dist<Rl, Rl, DIST_R_BIG>, DIST_R_BIG, sm);
     b->smem = sm;
     b->elig = dl;
     b->elig16 = ncl16 > 0 ? dl16 : std::vector<int>();
@@ -1009,6 +1069,40 @@ void luna_b200_plan_destroy(luna_plan* p) {
     delete p;
 }
 
+// CTAs of one FP64 right-hand side: the largest cluster that leaves each CTA 512 samples or sample
+// pairs (one launch has the GPU to itself, and what bounds it is the length of a CTA's loops); 1
+// where the distributed form does not apply.
+static int rhs_cluster(const LunaInst& I) {
+    LunaInst c = I;
+    c.grad = nullptr;  // a gradient may come and go: checked at each launch
+    auto sm = [&](int R) { return (int)dist_smem_bytes(dist_len(c), sizeof(cpx<double>), R); };
+    if (dist_fits<double>(c, 16) && max_clusters(rhs_kernel_dist<16>, 16, sm(16)) > 0) return 16;
+    if (dist_fits<double>(c, 8) && max_clusters(rhs_kernel_dist<8>, 8, sm(8)) > 0) return 8;
+    if (dist_fits<double>(c, 4) && max_clusters(rhs_kernel_dist<4>, 4, sm(4)) > 0) return 4;
+    return 1;
+}
+
+extern "C++" {
+template <int R>
+int launch_rhs_dist(luna_plan* p, const double2* Ew, double2* nl, cudaStream_t st, const TwDev& tw) {
+    const int sm = (int)dist_smem_bytes(dist_len(p->proto), sizeof(cpx<double>), R);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = R;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(R, 1, 1);
+    cfg.blockDim = dim3(LUNA_BLOCK, 1, 1);
+    cfg.dynamicSmemBytes = sm;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    CK(cudaLaunchKernelEx(&cfg, rhs_kernel_dist<R>, (const LunaInst*)p->d_inst, Ew, nl, tw.d, p->d_status));
+    return LUNA_OK;
+}
+}  // extern "C++"
+
 static int launch_rhs(luna_plan* p, const double2* Ew, double2* nl, cudaStream_t st, double z) {
     TwDev tw;
     int rc = get_tw(tw);
@@ -1031,6 +1125,12 @@ static int launch_rhs(luna_plan* p, const double2* Ew, double2* nl, cudaStream_t
     }
     const int maxs = max_smem_optin();
     if (p->precision == LUNA_PREC_FP64) {
+        if (!p->rhs_R) p->rhs_R = rhs_cluster(p->proto);
+        if (p->rhs_R > 1 && !p->proto.grad) {
+            const int R = p->rhs_R;
+            return R == 16 ? launch_rhs_dist<16>(p, Ew, nl, st, tw) : R == 8 ? launch_rhs_dist<8>(p, Ew, nl, st, tw)
+                                                                             : launch_rhs_dist<4>(p, Ew, nl, st, tw);
+        }
         int sm = (int)std::min<size_t>(smem_wanted<double>(p->proto), (size_t)maxs);
         CK(cudaFuncSetAttribute(rhs_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
         rhs_kernel<double><<<1, LUNA_BLOCK, sm, st>>>(p->d_inst, Ew, nl, tw.d, sm, p->d_status, z);
