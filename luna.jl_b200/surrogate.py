@@ -55,6 +55,7 @@ def load():
     lib = ctypes.CDLL(LIB_PATH)
     vp, i, ll, f, d = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float, ctypes.c_double
     lib.luna_sg_linear_fwd.argtypes = [vp, ll, vp, vp, i, i, i, i, vp, vp, vp, i, vp, vp]
+    lib.luna_sg_linear_ensemble.argtypes = [vp, ll, vp, vp, i, i, i, i, vp, vp, i, vp, vp]
     lib.luna_sg_linear_bwd_data.argtypes = [vp, vp, vp, i, i, i, vp, i, vp, vp]
     lib.luna_sg_linear_bwd_weight.argtypes = [vp, vp, ll, i, i, i, vp, vp, i, vp, vp]
     lib.luna_sg_features.argtypes = [vp, i, vp, i, vp, i, vp]
@@ -181,7 +182,6 @@ class Ensemble:
             m = self.members
             d = {"feat": t.empty(B, NIN, dtype=bf, device=self.dev),
                  "A": [t.empty(m, B, n, dtype=bf, device=self.dev) for n in WIDTHS[1:-1]],
-                 "Y": t.empty(m, B, NOUT, device=self.dev),
                  "loss": t.zeros(m, dtype=t.float64, device=self.dev)}
             if train:
                 d["Z"] = [t.empty(m, B, n, dtype=bf, device=self.dev) for n in WIDTHS[1:-1]]
@@ -189,29 +189,41 @@ class Ensemble:
             self._bufs[(B, train)] = d
         return self._bufs[(B, train)]
 
+    def _out(self, bf, B):
+        """The members' outputs of a forward pass (not needed by ``predict``)."""
+        if "Y" not in bf:
+            bf["Y"] = self.torch.empty(self.members, B, NOUT, device=self.dev)
+        return bf["Y"]
+
     @staticmethod
     def _p(x):
         return ctypes.c_void_p(x.data_ptr()) if x is not None else None
 
-    def forward(self, x, B=None, keep=True):
-        """Outputs [members, B, 768] FP32 for standardised inputs x [B, 8] (FP32 tensor);
-        ``keep`` stores the pre-activations a backward pass needs."""
+    def _layers(self, x, B, bf, keep, count, st):
+        """Features and the first ``count`` layers; the input of the next one and its member
+        stride."""
         lib, p = load(), self._p
-        B = x.shape[0] if B is None else B
-        bf = self._buf(B, keep)
-        st = ctypes.c_void_p(self.torch.cuda.current_stream().cuda_stream)
         _check(lib.luna_sg_features(p(x), B, p(self.fourier), NFOURIER, p(bf["feat"]), NIN, st), "features")
         X, sX = bf["feat"], 0
         nl = len(WIDTHS) - 1
-        for l in range(nl):
+        for l in range(count):
             K, N = WIDTHS[l], WIDTHS[l + 1]
             last = l == nl - 1
             _check(lib.luna_sg_linear_fwd(p(X), sX, p(self.Wb[l]), p(self.b[l]), B, K, N, 0 if last else 1,
                                           None if last else p(bf["A"][l]),
                                           None if (last or not keep) else p(bf["Z"][l]),
-                                          p(bf["Y"]) if last else None, self.members, p(self.err), st), "fwd")
+                                          p(self._out(bf, B)) if last else None, self.members, p(self.err), st), "fwd")
             if not last:
                 X, sX = bf["A"][l], B * N
+        return X, sX
+
+    def forward(self, x, B=None, keep=True):
+        """Outputs [members, B, 768] FP32 for standardised inputs x [B, 8] (FP32 tensor);
+        ``keep`` stores the pre-activations a backward pass needs."""
+        B = x.shape[0] if B is None else B
+        bf = self._buf(B, keep)
+        st = ctypes.c_void_p(self.torch.cuda.current_stream().cuda_stream)
+        self._layers(x, B, bf, keep, len(WIDTHS) - 1, st)
         return bf["Y"]
 
     def train_step(self, x, T):
@@ -250,14 +262,23 @@ class Ensemble:
     def predict(self, x):
         """Ensemble mean [B, 768] and spread [B] (largest member standard deviation over the
         spectral outputs, in decades) for standardised inputs x [B, 8]."""
-        lib, p, t = load(), self._p, self.torch
+        t = self.torch
         B = x.shape[0]
-        Y = self.forward(x, B, keep=False)
         mean = t.empty(B, NOUT, device=self.dev)
         spread = t.empty(B, device=self.dev)
-        _check(lib.luna_sg_ensemble(p(Y), self.members, B, NOUT, NSPEC, p(mean), p(spread),
-                                    ctypes.c_void_p(t.cuda.current_stream().cuda_stream)), "ensemble")
+        self._predict_into(x, mean, spread)
         return mean, spread
+
+    def _predict_into(self, x, mean, spread):
+        """``predict`` into given tensors: the last layer leaves its ensemble statistics instead
+        of the members' outputs."""
+        lib, p = load(), self._p
+        B = x.shape[0]
+        bf = self._buf(B, False)
+        st = ctypes.c_void_p(self.torch.cuda.current_stream().cuda_stream)
+        X, sX = self._layers(x, B, bf, False, len(WIDTHS) - 2, st)
+        _check(lib.luna_sg_linear_ensemble(p(X), sX, p(self.Wb[-1]), p(self.b[-1]), B, WIDTHS[-2], NOUT, NSPEC, p(mean),
+                                           p(spread), self.members, p(self.err), st), "ensemble")
 
     def check_timeout(self):
         if int(self.err.item()) != 0:
@@ -410,17 +431,24 @@ def predict(model, x, chunk=1 << 17):
     to a multiple of 128 internally."""
     import torch
     n = x.shape[0]
-    means, spreads = [], []
+    n128 = (n + 127) // 128 * 128
+    if n == 0 or chunk <= 0 or chunk % 128:  # chunks that each need padding (or none)
+        means, spreads = [], []
+        for c0 in range(0, n, chunk):
+            mu, sp = predict(model, x[c0:c0 + chunk], (chunk + 127) // 128 * 128)
+            means.append(mu)
+            spreads.append(sp)
+        return torch.cat(means), torch.cat(spreads)
+    mean = torch.empty(n128, NOUT, device=model.dev)
+    spread = torch.empty(n128, device=model.dev)
     for c0 in range(0, n, chunk):
         xc = x[c0:c0 + chunk]
         m = xc.shape[0]
         pad = (-m) % 128
         if pad:
             xc = torch.cat([xc, xc[:1].expand(pad, -1)])
-        mu, sp = model.predict(xc.contiguous())
-        means.append(mu[:m])
-        spreads.append(sp[:m])
-    return torch.cat(means), torch.cat(spreads)
+        model._predict_into(xc.contiguous(), mean[c0:c0 + m + pad], spread[c0:c0 + m + pad])
+    return mean[:n], spread[:n]
 
 
 def spectral_error(pred, true):
