@@ -909,9 +909,10 @@ __device__ __forceinline__ void dist_rhs(const LunaInst& I, DWs<Rl>& d, LoadF&& 
 template <typename Rl, typename Kt, int R>
 __device__ __noinline__ void solve_instance_dist(LunaInst& I, DWs<Rl>& d, Ctl& c) {
     const int p = d.rank, T = LUNA_BLOCK, tid = threadIdx.x;
-    const int Nw = I.Nw, Mcoarse = I.N / 2;
+    const int Nw = I.Nw, M = I.No / 2, Mcoarse = I.N / 2;
     const bool writer = (p == 0);
     const cpx<double>* L = reinterpret_cast<const cpx<double>*>(I.linop);
+    const cpx<double>* of = reinterpret_cast<const cpx<double>*>(I.outfac);
     void** k = c.k;
     if (tid == 0) {
         for (int j = 0; j < 7; ++j) k[j] = I.k[j];
@@ -942,7 +943,18 @@ __device__ __noinline__ void solve_instance_dist(LunaInst& I, DWs<Rl>& d, Ctl& c
         }
     }
     __syncthreads();
-    auto rhs_d = [&](auto&& load, auto&& store) { dist_rhs<Rl, R>(I, d, load, store); };
+    const double sc = I.in_scale;
+    auto rhs_d = [&](auto&& load, auto&& store) {
+        if constexpr (sizeof(Rl) == 8) {
+            dist_rhs<Rl, R>(I, d, load, store);
+        } else {
+            // written out: which products of load's and store's FP64 expressions the compiler
+            // fuses follows the nesting, and a fused one can flip the FP32 rounding after it
+            dist_c2r<Rl, R>(d, M, Nw, load);
+            dist_pointwise<Rl, R>(I, d, M, sc);
+            dist_r2c<Rl, R>(d, M, Nw, [&](int kb, cpx<double> X) { store(kb, X * ldg(of + kb)); });
+        }
+    };
     {
         const cpx<double>* y = reinterpret_cast<const cpx<double>*>(py);
         void* k0 = k[0];
@@ -1076,13 +1088,14 @@ __device__ __noinline__ void solve_instance_dist(LunaInst& I, DWs<Rl>& d, Ctl& c
             {
                 cpx<double>* Yo = reinterpret_cast<cpx<double>*>(pyn);
                 const double inv = 1.0 / (double)I.N;
-                auto win = [&](int i) -> cpx<double> { return scale(__ldg(I.wwin + i), Yo[i] * e1[i]); };
                 bool env = false;
                 if constexpr (sizeof(Rl) == 8) {
                     env = I.kind == 1;
                     if (env) {
                         const int Mb = I.N / R;
-                        dist_c2c_inv<R>(d, I.N, win);
+                        dist_c2c_inv<R>(d, I.N, [&](int i) -> cpx<double> {
+                            return scale(__ldg(I.wwin + i), Yo[i] * e1[i]);
+                        });
                         for (int n1 = tid; n1 < Mb; n1 += T) {
                             const int pos = Swz<double>::f(n1);
                             d.tb[pos] = scale(inv * __ldg(I.twin + p * Mb + n1), d.tb[pos]);
@@ -1092,7 +1105,9 @@ __device__ __noinline__ void solve_instance_dist(LunaInst& I, DWs<Rl>& d, Ctl& c
                     }
                 }
                 if (!env) {
-                dist_c2r<Rl, R>(d, Mcoarse, Nw, win);
+                dist_c2r<Rl, R>(d, Mcoarse, Nw, [&](int i) -> cpx<double> {
+                    return scale(__ldg(I.wwin + i), Yo[i] * e1[i]);
+                });
                 const int Mbc = Mcoarse / R;
                 for (int n1 = tid; n1 < Mbc; n1 += T) {
                     const int pos = Swz<Rl>::f(n1);
