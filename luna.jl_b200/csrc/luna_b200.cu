@@ -2210,6 +2210,9 @@ struct luna_modal_plan {
     void* Et = nullptr;  // [Nr*No/2] field samples per mode
     void* G = nullptr;   // [nslots*Nr*No/2] projected polarisation per node
     double* vscr = nullptr;  // two components with plasma: [6*No] doubles per node CTA
+    int R = 0, C = 0;        // modal_dist_kernel: CTAs of a cluster (0: the kernels of one CTA) and clusters
+    bool elem = false;       // Kerr responses alone
+    ModalBar* bar = nullptr;
     bool vplasma = false;
     ModalState* ms = nullptr;
     int* d_flags = nullptr;
@@ -2242,10 +2245,59 @@ ModalArgs modal_args(const luna_modal_plan* p, const RadState* st) {
     return a;
 }
 
+template <int R>
+int launch_modal_dist(luna_modal_plan* p, const double2* src, double2* dst, const TwTab<double>& tw, RadState* st,
+                      int* flags, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = R;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeCooperative;  // clusters that wait for one another
+    at[1].val.cooperative = 1;
+    cfg.gridDim = dim3(R * p->C, 1, 1);
+    cfg.blockDim = dim3(LUNA_BLOCK, 1, 1);
+    cfg.dynamicSmemBytes = dist_smem_bytes(p->Mt, sizeof(cpx<double>), R);
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = p->C > 1 ? 2 : 1;
+    CK(cudaLaunchKernelEx(&cfg, modal_dist_kernel<R>, (const LunaInst*)p->d_col, src, modal_args(p, st), (double2*)p->B, dst,
+                          (int)p->elem, tw, flags, p->bar));
+    return LUNA_OK;
+}
+
+// src: the stage input; dst: the right-hand side with its output factor (null: only B)
+int modal_dist(luna_modal_plan* p, const double2* src, double2* dst, const TwTab<double>& tw, RadState* st, int* flags,
+               cudaStream_t s) {
+    switch (p->R) {
+        case 16: return launch_modal_dist<16>(p, src, dst, tw, st, flags, s);
+        case 8: return launch_modal_dist<8>(p, src, dst, tw, st, flags, s);
+        default: return launch_modal_dist<4>(p, src, dst, tw, st, flags, s);
+    }
+}
+
+// Clusters of a plan: full precision, time buffers that give each CTA of a cluster 512
+// samples, and not the two-component plasma (its scans run on one CTA a node). As many clusters as
+// modes (Kerr alone: 33 us at No = 16384 with one mode, 330 us with the kernels of one CTA) or as nodes of
+// the third refinement, if that many are resident together.
+template <int R>
+bool modal_dist_setup(luna_modal_plan* p) {
+    const LunaInst& I = p->col->proto;
+    if (!dist_fits<double>(I, R)) return false;
+    const int most = max_clusters(modal_dist_kernel<R>, R, (int)dist_smem_bytes(p->Mt, sizeof(cpx<double>), R));
+    if (most < 1) return false;
+    p->R = R;
+    p->C = std::min(most, p->elem ? p->Nr : std::max(p->Nr, 1 << std::min(p->nlevels - 1, 3)));
+    return true;
+}
+
 // Transform of the stage input in A into B: fields per mode, then for each cubature level
 // its new nodes and its integral; levels after convergence return at once.
 template <typename Rl>
 int modal_xform(luna_modal_plan* p, const TwTab<Rl>& tw, RadState* st, int* flags, cudaStream_t s) {
+    if constexpr (sizeof(Rl) == 8)
+        if (p->R) return modal_dist(p, (const double2*)p->A, nullptr, tw, st, flags, s);
     const ModalArgs a = modal_args(p, st);
     modal_time_kernel<Rl><<<p->Nr, LUNA_BLOCK, p->smem, s>>>(p->d_col, (const cpx<Rl>*)p->A, a, tw, p->smem, p->gscr,
                                                              p->gstride);
@@ -2289,6 +2341,14 @@ int modal_setup(luna_modal_plan* p) {
     // the largest level has 2^(nlevels - 1) new nodes, one CTA each
     if (p->vplasma && dalloc(p->allocs, &p->vscr, sizeof(double) * 6 * (size_t)I.No * ((size_t)1 << (p->nlevels - 1))))
         return LUNA_ERR_CUDA;
+    if constexpr (sizeof(Rl) == 8) {
+        if (!p->vplasma) {
+            p->elem = true;
+            for (int i = 0; i < I.nresp; ++i)
+                p->elem = p->elem && (I.resp[i].kind == LUNA_RESP_KERR_FIELD || I.resp[i].kind == LUNA_RESP_KERR_ENV);
+            if (!modal_dist_setup<16>(p) && !modal_dist_setup<8>(p)) modal_dist_setup<4>(p);
+        }
+    }
     CK(cudaFuncSetAttribute(modal_time_kernel<Rl>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs));
     CK(cudaFuncSetAttribute(modal_node_kernel<Rl>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs));
     CK(cudaFuncSetAttribute(modal_level_kernel<Rl>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs));
@@ -2305,7 +2365,9 @@ int modal_rhs(luna_modal_plan* p, const double2* Ew, double2* nl, cudaStream_t s
     const TwTab<Rl>& t = *reinterpret_cast<const TwTab<Rl>*>(std::is_same<Rl, double>::value ? (const void*)&tw.d : (const void*)&tw.f);
     RadArgs a{p->Nw, p->Nr, nullptr, p->outfac, nullptr, nullptr};
     const size_t n = (size_t)p->Nw * p->Nr;
-    CK(cudaMemsetAsync(p->d_flags, 0, sizeof(int), s));
+    CK(cudaMemsetAsync(p->d_flags, 0, sizeof(int) + sizeof(ModalBar), s));
+    if constexpr (sizeof(Rl) == 8)
+        if (p->R) return modal_dist(p, Ew, nl, t, nullptr, p->d_flags, s);
     rad_stage_kernel<Rl, double><<<rad_grid(n), 256, 0, s>>>(a, -1, Ew, (cpx<Rl>*)p->A);
     modal_xform<Rl>(p, t, nullptr, p->d_flags, s);
     rad_store_kernel<Rl, double><<<rad_grid(n), 256, 0, s>>>(a, -1, (const cpx<Rl>*)p->B, nl);
@@ -2387,10 +2449,12 @@ int luna_b200_modal_plan_create(const luna_grid_desc* g, const luna_resp_desc* r
         return bail(LUNA_ERR_CUDA);
     p->outfac = (const double2*)tmp;
     const size_t cb = sizeof(double2);
-    if (dalloc(p->allocs, &p->A, cb * n) || dalloc(p->allocs, &p->B, cb * n) || dalloc(p->allocs, &p->d_flags, sizeof(int)) ||
-        dalloc(p->allocs, &p->ms, sizeof(ModalState)) || dalloc(p->allocs, &p->d_col, sizeof(LunaInst)))
+    if (dalloc(p->allocs, &p->A, cb * n) || dalloc(p->allocs, &p->B, cb * n) ||
+        dalloc(p->allocs, &p->d_flags, sizeof(int) + sizeof(ModalBar)) || dalloc(p->allocs, &p->ms, sizeof(ModalState)) || dalloc(p->allocs, &p->d_col, sizeof(LunaInst)))
         return bail(LUNA_ERR_CUDA);
+    p->bar = reinterpret_cast<ModalBar*>(p->d_flags + 1);
     if (cudaMemset(p->ms, 0, sizeof(ModalState)) != cudaSuccess ||
+        cudaMemset(p->d_flags, 0, sizeof(int) + sizeof(ModalBar)) != cudaSuccess ||
         cudaMemcpy(p->d_col, &col->proto, sizeof(LunaInst), cudaMemcpyHostToDevice) != cudaSuccess)
         return bail(fail(LUNA_ERR_CUDA, "modal_plan_create: initialising the device state failed"));
     rc = (precision == LUNA_PREC_FP64) ? modal_setup<double>(p) : modal_setup<float>(p);
@@ -2432,6 +2496,7 @@ int luna_b200_modal_rhs(luna_modal_plan* p, double* nl, const double* Ew, double
     CK(cudaMemcpyAsync(&nev, &p->ms->nevals, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
     CK(cudaStreamSynchronize(p->stream));
     if (nevals) *nevals = nev;
+    if (fl & (1 << ST_WAIT_TIMEOUT)) return fail(LUNA_WAIT_TIMEOUT, "modal_rhs: the wait of a cluster for the others timed out");
     if (fl & (1 << ST_FIELD_ABOVE_EMAX)) return fail(LUNA_FIELD_ABOVE_EMAX, "Field strength exceeds maximum for PPT ionisation rate.");
     return LUNA_OK;
 }
@@ -2440,6 +2505,8 @@ int luna_b200_modal_solve(luna_modal_plan* p, const double* linop, double* y_ino
                           const luna_solve_opts* opts, double* saves, double* steplog, luna_solve_stats* stats) {
     if (!p || !linop || !y_inout || !opts) return fail(LUNA_ERR_BAD_ARG, "modal_solve: null argument");
     if (opts->saveN < 0 || (opts->saveN > 0 && !opts->zsave)) return fail(LUNA_ERR_BAD_ARG, "modal_solve: save points missing");
+    // a solve that ended in a timed-out wait leaves the barrier's count behind
+    CK(cudaMemset(p->bar, 0, sizeof(ModalBar)));
     if (p->precision == LUNA_PREC_FP64)
         return col_solve<double, double>(
             p, [p](const TwTab<double>& t, RadState* st, int* fl, cudaStream_t s) { return modal_xform<double>(p, t, st, fl, s); },

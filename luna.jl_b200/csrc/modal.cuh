@@ -23,6 +23,7 @@
 // holds the sample pair n with Swz(split_pos(n)) == i), the same in every kernel, so node
 // and level sums are plain element-wise loops over the buffers.
 #pragma once
+#include "dist.cuh"
 #include "radial.cuh"
 
 namespace luna {
@@ -37,6 +38,7 @@ struct ModalState {
     int pad;
     double err;       // L2 error estimate of the last level
     double part[2 * MODAL_MAX_MODES];  // per mode: sum |F_l - F_{l-1}|^2, sum |F_l|^2
+    double part1[2 * MODAL_MAX_MODES]; // the same of the odd levels (modal_dist_kernel)
 };
 
 struct ModalArgs {
@@ -414,6 +416,238 @@ modal_level_kernel(const LunaInst* inst, ModalArgs a, int l, cpx<Rl>* B, TwTab<R
             ms->ticket = 0;
         }
     }
+}
+
+// ------------------------------------------------------------------ one launch on clusters (FP64)
+// The whole transform in one launch, for time buffers from 2048 samples: clusters of R CTAs
+// (the largest of 16, 8 and 4 that leaves 512 samples a CTA) take a mode's or a node's
+// time samples together, as a distributed right-hand side does (dist.cuh). Time samples are in natural
+// order, CTA q holding the block q. The kernels above run one CTA a mode, 17 to 19 launches of which
+// those after convergence do nothing: at No = 16384 with one mode and 15 nodes 25 us for the field,
+// 31 us for each level's nodes and 56 to 100 us for its integral. Bound by the chain of one transform
+// per level.
+//
+// elem (Kerr responses alone): the integrand is local in time, so each level's sum over its nodes
+// is evaluated in registers from the mode fields, without G; nothing but the convergence
+// test crosses modes, and one mode needs a single cluster. Otherwise clusters take the new nodes of a
+// level, leave the projections in G, and after a grid barrier sum them per mode. Several clusters are
+// a cooperative launch: all are resident, and modal_gsync bounds its wait besides.
+struct ModalBar {
+    unsigned count, gen;
+};
+
+// Barrier of all clusters of the grid (C = 1: of the cluster). False when the wait ran out; every
+// thread of a cluster returns the same.
+template <int R>
+__device__ __forceinline__ bool modal_gsync(DWs<double>& d, ModalBar* bar, int C) {
+    dsync();
+    if (C == 1) return true;
+    if (d.rank == 0 && threadIdx.x == 0) {
+        volatile unsigned* vg = &bar->gen;
+        const unsigned g = *vg;
+        bool ok = true;
+        __threadfence();
+        if (atomicAdd(&bar->count, 1u) == (unsigned)C - 1) {
+            bar->count = 0;
+            __threadfence();
+            *vg = g + 1;
+        } else {
+            unsigned n = 0;
+            while (*vg == g && ++n < (1u << 24)) __nanosleep(20);
+            ok = n < (1u << 24);
+        }
+        __threadfence();
+        d.xs[15] = ok ? 1.0 : 0.0;
+    }
+    dsync();
+    return *drem(&d.xs[15], 0) != 0.0;
+}
+
+// Polarisation of one slot (a sample pair, or a complex sample on an envelope grid) of a node
+// times e_c, Kerr responses only, without the time window: the expressions of modal_node_kernel
+// and modal_kerr2_kernel. f holds the components of the node's field.
+__device__ __forceinline__ cpx<double> modal_kerr(const LunaInst& I, int npol, double kc, int n, cpx<double> fx,
+                                                  cpx<double> fy, double ex, double ey) {
+    if (I.kind == 0) {
+        if (npol == 1) return mk<double>(ex * (kc * (fx.x * fx.x * fx.x)), ex * (kc * (fx.y * fx.y * fx.y)));
+        const double k0 = kc * (fx.x * fx.x + fy.x * fy.x), k1 = kc * (fx.y * fx.y + fy.y * fy.y);
+        return mk<double>(ex * (k0 * fx.x) + ey * (k0 * fy.x), ex * (k1 * fx.y) + ey * (k1 * fy.y));
+    }
+    if (npol == 1) {
+        cpx<double> P = mk<double>(0, 0);
+        for (int i = 0; i < I.nresp; ++i) {
+            const LunaResp& r = I.resp[i];
+            if (r.cthg) {
+                const cpx<double> C = ldg(reinterpret_cast<const cpx<double>*>(r.cthg) + n);
+                P = P + scale(0.25 * r.coef, scale(3.0 * abs2(fx), fx) + C * (fx * fx) * fx);
+            } else {
+                P = P + scale(0.75 * r.coef * abs2(fx), fx);
+            }
+        }
+        return scale(ex, P);
+    }
+    const double ax = abs2(fx), ay = abs2(fy), f = 0.75 * kc;
+    const cpx<double> px = scale(f, scale(ax + 2.0 / 3 * ay, fx) + scale(1.0 / 3, conj(fx) * (fy * fy)));
+    const cpx<double> py = scale(f, scale(ay + 2.0 / 3 * ax, fy) + scale(1.0 / 3, conj(fy) * (fx * fx)));
+    return scale(ex, px) + scale(ey, py);
+}
+
+template <int R>
+__global__ void __launch_bounds__(LUNA_BLOCK, 1)
+modal_dist_kernel(const LunaInst* inst, const double2* A, ModalArgs a, double2* B, double2* dst, int elem,
+                  TwTab<double> tw, int* flags, ModalBar* bar) {
+    if (a.st && a.st->finished) return;
+    __shared__ LunaInst sI;
+    __shared__ int s_done;
+    tws_fill(tw);
+    const LunaInst& I = local_inst<double>(inst, &sI);
+    DWs<double> d;
+    plan_dws<double, R>(I, dsm, d, tw, (int)cooperative_groups::this_cluster().block_rank());
+    const int tid = threadIdx.x, T = LUNA_BLOCK, p = d.rank;
+    const int C = gridDim.x / R, cl = blockIdx.x / R;
+    const int Mt = a.Mt, Mb = Mt / R, base = p * Mb, nm = a.nmodes, np = a.npol, Nw = I.Nw;
+    const int No = I.No, N = I.N, h = I.N / 2;  // envelope grids: copy_scale_both! padding and cropping
+    const double sc = I.in_scale;
+    cpx<double>* Et = reinterpret_cast<cpx<double>*>(a.Et);
+    cpx<double>* G = reinterpret_cast<cpx<double>*>(a.G);
+    if (tid == 0) *d.flag = 0;
+    dsync();  // every CTA of the cluster has started before its shared memory is addressed
+    for (int m = cl; m < nm; m += C) {
+        const cpx<double>* E = reinterpret_cast<const cpx<double>*>(A) + (size_t)m * Nw;
+        if (I.kind == 1)
+            dist_c2c_inv<R>(d, No, [&](int j) { return j < h ? E[j] : j >= No - h ? E[j - No + N] : mk<double>(0, 0); });
+        else
+            dist_c2r<double, R>(d, No / 2, Nw, [&](int k) { return E[k]; });
+        for (int n = tid; n < Mb; n += T) Et[(size_t)m * Mt + base + n] = d.tb[Swz<double>::f(n)];
+    }
+    bool ok = modal_gsync<R>(d, bar, C);
+    for (int l = 0; ok; ++l) {
+        const int ns = (2 << l) - 1;  // interior nodes of level l
+        if (!elem) {
+            const int s0 = (l == 0) ? 0 : (1 << l) - 1, nn = (l == 0) ? 1 : (1 << l);
+            for (int s = s0 + cl; s < s0 + nn; s += C) {
+                const double* e = a.ems + (size_t)s * nm;
+                for (int n = tid; n < Mb; n += T) {
+                    cpx<double> f = mk<double>(0, 0);
+                    for (int m = 0; m < nm; ++m) f = f + scale(__ldg(e + m), Et[(size_t)m * Mt + base + n]);
+                    d.tb[Swz<double>::f(n)] = f;
+                }
+                __syncthreads();
+                if (I.kind == 1) dist_pointwise_env<R>(I, d, sc);
+                else dist_pointwise<double, R>(I, d, Mt, sc);
+                for (int n = tid; n < Mb; n += T) {
+                    const cpx<double> v = d.tb[Swz<double>::f(n)];
+                    for (int m = 0; m < nm; ++m) G[((size_t)s * nm + m) * Mt + base + n] = scale(__ldg(e + m), v);
+                }
+                dsync();  // the blocks may be written again
+            }
+            if (!(ok = modal_gsync<R>(d, bar, C))) break;
+        }
+        const double* wl = a.wts + (size_t)l * a.nslots;
+        // level 0 has one node: one transform gives its rule and the midpoint rule's value
+        const double w0 = l == 0 ? 1.0 : 0.0, wa = l == 0 ? a.wlow : 0.0, wb = l == 0 ? __ldg(wl) : 1.0;
+        ModalState* ms = a.ms;
+        double* part = (l & 1) ? ms->part1 : ms->part;
+        for (int c = cl; c < nm; c += C) {
+            for (int n = tid; n < Mb; n += T) {
+                cpx<double> x = mk<double>(0, 0);
+                if (elem) {
+                    cpx<double> v[4];
+#pragma unroll
+                    for (int m = 0; m < 4; ++m)
+                        if (m < nm) v[m] = Et[(size_t)m * Mt + base + n];
+#pragma unroll 2
+                    for (int s = 0; s < ns; ++s) {
+                        const double* e = a.ems + (size_t)s * nm * np;
+                        cpx<double> fx = mk<double>(0, 0), fy = fx;
+#pragma unroll
+                        for (int m = 0; m < 4; ++m) {
+                            if (m >= nm) break;
+                            fx = fx + scale(__ldg(e + m * np), v[m]);
+                            if (np == 2) fy = fy + scale(__ldg(e + m * np + 1), v[m]);
+                        }
+                        for (int m = 4; m < nm; ++m) {
+                            const cpx<double> u = Et[(size_t)m * Mt + base + n];
+                            fx = fx + scale(__ldg(e + m * np), u);
+                            if (np == 2) fy = fy + scale(__ldg(e + m * np + 1), u);
+                        }
+                        const double ey = np == 2 ? __ldg(e + c * np + 1) : 0.0;
+                        const cpx<double> P = modal_kerr(I, np, a.kerr, base + n, scale(sc, fx), scale(sc, fy), __ldg(e + c * np), ey);
+                        x = x + scale(l == 0 ? w0 : __ldg(wl + s), P);
+                    }
+                    if (I.kind == 1) {
+                        x = scale(__ldg(I.towin + base + n), x);
+                    } else {
+                        const double2 t = __ldg(reinterpret_cast<const double2*>(I.towin) + base + n);
+                        x = mk<double>(x.x * t.x, x.y * t.y);
+                    }
+                } else {
+#pragma unroll 4
+                    for (int s = 0; s < ns; ++s)
+                        x = x + scale(l == 0 ? w0 : __ldg(wl + s), G[((size_t)s * nm + c) * Mt + base + n]);
+                }
+                d.tb[Swz<double>::f(n)] = x;
+            }
+            cpx<double>* Bc = reinterpret_cast<cpx<double>*>(B) + (size_t)c * Nw;
+            const cpx<double>* of = reinterpret_cast<const cpx<double>*>(a.outfac) + (size_t)c * Nw;
+            double se = 0, sv = 0;
+            auto st = [&](int k, cpx<double> X) {
+                const cpx<double> o = ldg(of + k), last = l == 0 ? scale(wa, X) : Bc[k];
+                X = scale(wb, X);
+                se += abs2((X - last) * o);
+                sv += abs2(X * o);
+                Bc[k] = X;
+            };
+            if (I.kind == 1)
+                dist_c2c_fwd<R>(d, No, [&](int j, cpx<double> X) { if (j < h || j >= No - h) st(j < h ? j : j - No + N, X); });
+            else
+                dist_r2c<double, R>(d, Mt, Nw, st);
+            double unused = 0;
+            block_sum3(se, sv, unused, d.red);
+            if (tid == 0) {
+                d.xs[8] = se;
+                d.xs[9] = sv;
+            }
+            dsync();
+            if (p == 0 && tid == 0) {
+                double e2 = 0, v2 = 0;
+                for (int j = 0; j < R; ++j) {
+                    const double* x = drem(d.xs, j);
+                    e2 += x[8];
+                    v2 += x[9];
+                }
+                part[2 * c] = e2;
+                part[2 * c + 1] = v2;
+            }
+        }
+        if (!(ok = modal_gsync<R>(d, bar, C))) break;
+        if (tid == 0) {  // every CTA adds the same sums in the same order: identical decisions
+            double e2 = 0, v2 = 0;
+            for (int m = 0; m < nm; ++m) {
+                e2 += __ldcg(part + 2 * m);
+                v2 += __ldcg(part + 2 * m + 1);
+            }
+            const double err = sqrt(e2), val = sqrt(v2);
+            s_done = err <= a.atol || err <= a.rtol * val || l >= a.lmax;
+            if (blockIdx.x == 0) {
+                ms->err = err;
+                ms->nevals = (2 << l) + 1;
+            }
+        }
+        __syncthreads();
+        if (s_done) break;
+    }
+    if (!ok && tid == 0) atomicOr(flags, 1 << ST_WAIT_TIMEOUT);
+    if (ok && dst) {
+        for (int c = cl; c < nm; c += C)
+            for (int k = p + R * tid; k < Nw; k += R * T) {
+                const size_t e = (size_t)c * Nw + k;
+                const cpx<double> X = reinterpret_cast<const cpx<double>*>(B)[e] * ldg(reinterpret_cast<const cpx<double>*>(a.outfac) + e);
+                dst[e] = make_double2(X.x, X.y);
+            }
+    }
+    if (tid == 0 && *d.flag) atomicOr(flags, *d.flag);
+    dsync();  // no CTA leaves while another may read its shared memory
 }
 
 }  // namespace luna
