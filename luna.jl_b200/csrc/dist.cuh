@@ -102,6 +102,37 @@ __device__ __forceinline__ cpx<Rl> tw_pow(const TwTab<Rl>& tw, unsigned a, int l
     return twiddle<Rl, INV>(tw, (a & ((1u << lg) - 1)) << (TW_LOG_MMAX - lg));
 }
 
+// FP64 exp(-+2 pi i a / 4096), a < 2048, from the table in shared memory
+template <bool INV>
+__device__ __forceinline__ cpx<double> tws_half(int a) {
+    cpx<double> w = tws_get<double, false>(a & 1023);
+    if (a & 1024) w = mk<double>(w.y, -w.x);
+    return INV ? conj(w) : w;
+}
+
+// Cluster barrier, then buf[n1] *= exp(-+2 pi i f n1 / 2^lg) for this CTA's sub-transform f: the
+// twiddles of the FP64 radix steps on the receiving side, one a thread. The CTAs that form the
+// steps have 32 threads at work (Mb = 512, R = 16), and their R - 1 lookups between remote stores took
+// 8 k of the 21 k cycles of a 16384-point transform. (A DFT over R lanes of a warp, on every thread,
+// loses that again to remote accesses of R different CTAs in one instruction.)
+__device__ __forceinline__ void dsync_twiddle(const TwTab<double>& tw, cpx<double>* b0, int f0, cpx<double>* b1, int f1,
+                                              int Mb, int lg) {
+    const int tid = threadIdx.x;
+    cpx<double> w0 = tw_pow<double, false>(tw, (unsigned)(f0 * tid), lg);
+    cpx<double> w1 = b1 ? tw_pow<double, false>(tw, (unsigned)(f1 * tid), lg) : w0;
+    dsync();
+    for (int n1 = tid; n1 < Mb; n1 += LUNA_BLOCK) {
+        const int pos = Swz<double>::f(n1);
+        if (n1 != tid) {
+            w0 = tw_pow<double, false>(tw, (unsigned)(f0 * n1), lg);
+            if (b1) w1 = tw_pow<double, false>(tw, (unsigned)(f1 * n1), lg);
+        }
+        if (f0) b0[pos] = b0[pos] * w0;
+        if (b1) b1[pos] = b1[pos] * w1;
+    }
+    __syncthreads();
+}
+
 // Join of an inverse transform of R Mb points, transposed: this CTA takes the n1 of its slice
 // [p S, (p + 1) S), S = Mb/R, gathers B_r[n1] from every CTA's fb, forms
 // x[n1 + Mb q] = sum_r W_R^{-r q} B_r[n1] for every q with one in-register DFT and stores each
@@ -137,9 +168,13 @@ __device__ __forceinline__ void dist_radix(DWs<Rl>& d, int Mb, int lgM) {
         dft_br<Rl, false, R>(v);
         drem(d.fb, 0)[pos] = v[0];
 #pragma unroll
-        for (int r = 1; r < R; ++r) drem(d.fb, r)[pos] = v[r] * tw_pow<Rl, false>(d.tw, (unsigned)(r * n1), lgM);
+        for (int r = 1; r < R; ++r) {
+            if constexpr (sizeof(Rl) == 8) drem(d.fb, r)[pos] = v[r];
+            else drem(d.fb, r)[pos] = v[r] * tw_pow<Rl, false>(d.tw, (unsigned)(r * n1), lgM);
+        }
     }
-    dsync();
+    if constexpr (sizeof(Rl) == 8) dsync_twiddle(d.tw, d.fb, d.rank, (cpx<double>*)nullptr, 0, Mb, lgM);
+    else dsync();
 }
 
 // ------------------------------------------------------------------ real transform pair
@@ -320,6 +355,15 @@ __device__ __noinline__ void dist_raman_fwd(const LunaResp& rr, DWs<Rl>& d, cpx<
             }
             dft_br<Rl, false, R2>(v);
             drem(d.rb0, 0)[pos] = v[0];
+            if constexpr (sizeof(Rl) == 8) {
+                drem(d.rb1, 0)[pos] = v[R];
+#pragma unroll
+                for (int cc = 1; cc < R; ++cc) {
+                    drem(d.rb0, cc)[pos] = v[cc];
+                    drem(d.rb1, cc)[pos] = v[R2 - cc];
+                }
+                continue;
+            }
             drem(d.rb1, 0)[pos] = v[R] * tw_pow<Rl, false>(d.tw, (unsigned)(R * n1), lgMr);
 #pragma unroll
             for (int cc = 1; cc < R; ++cc) {
@@ -327,7 +371,8 @@ __device__ __noinline__ void dist_raman_fwd(const LunaResp& rr, DWs<Rl>& d, cpx<
                 drem(d.rb1, cc)[pos] = v[R2 - cc] * tw_pow<Rl, false>(d.tw, (unsigned)((R2 - cc) * n1), lgMr);
             }
         }
-        dsync();
+        if constexpr (sizeof(Rl) == 8) dsync_twiddle(d.tw, d.rb0, pa, d.rb1, pb, Mb, lgMr);
+        else dsync();
     } else {
         static_assert(R == 16, "cluster sizes: 4, 8, 16");
         // the same transposed step with the 2R-point DFT as two R-point ones (a 2R-point
@@ -351,19 +396,26 @@ __device__ __noinline__ void dist_raman_fwd(const LunaResp& rr, DWs<Rl>& d, cpx<
                     } else {
                         v[i] = ev;
                     }
-                    if (e && q) v[i] = v[i] * tw_pow<Rl, false>(d.tw, (unsigned)q, lg2R);
+                    if constexpr (sizeof(Rl) == 8) {
+                        if (e && q) v[i] = v[i] * tws_half<false>(q * (2048 / R));
+                    } else if (e && q) v[i] = v[i] * tw_pow<Rl, false>(d.tw, (unsigned)q, lg2R);
                 }
                 dft_br<Rl, false, R>(v);
 #pragma unroll
                 for (int g = 0; g < R; ++g) {
                     const int f = 2 * g + e;  // sub-transform f: rb0 of CTA f (f < R), rb1 of CTA 2R - f
+                    if constexpr (sizeof(Rl) == 8) {
+                        drem(f < R ? d.rb0 : d.rb1, f <= R ? f % R : 2 * R - f)[pos] = v[g];
+                        continue;
+                    }
                     if (f == 0) drem(d.rb0, 0)[pos] = v[g];
                     else if (f < R) drem(d.rb0, f)[pos] = v[g] * tw_pow<Rl, false>(d.tw, (unsigned)(f * n1), lgMr);
                     else drem(d.rb1, f == R ? 0 : 2 * R - f)[pos] = v[g] * tw_pow<Rl, false>(d.tw, (unsigned)(f * n1), lgMr);
                 }
             }
         }
-        dsync();
+        if constexpr (sizeof(Rl) == 8) dsync_twiddle(d.tw, d.rb0, pa, d.rb1, pb, Mb, lgMr);
+        else dsync();
     }
     fft_sub2<Rl, false>(d.rb0, d.rb1, Mb, d.tw);
     // pairs (f, Mr - f) with f = 2R k + p; Zk/Zm are entries of the complex transform
@@ -437,7 +489,9 @@ __device__ __forceinline__ void raman_out_scatter(DWs<Rl>& d, cpx<Rl>* out, int 
                     const int g = bitrev<R>(i);
                     const cpx<Rl> a = drem(d.rb0, g)[pos];                   // B_g
                     const cpx<Rl> b = drem(d.rb1, g == 0 ? 0 : R - g)[pos];  // B_{g+R}
-                    v[i] = e ? (g ? (a - b) * tw_pow<Rl, true>(d.tw, (unsigned)g, lg2R) : a - b) : a + b;
+                    if constexpr (sizeof(Rl) == 8)
+                        v[i] = e ? (g ? (a - b) * tws_half<true>(g * (2048 / R)) : a - b) : a + b;
+                    else v[i] = e ? (g ? (a - b) * tw_pow<Rl, true>(d.tw, (unsigned)g, lg2R) : a - b) : a + b;
                 }
                 dft_br<Rl, true, R>(v);
 #pragma unroll

@@ -463,13 +463,12 @@ __device__ __forceinline__ bool modal_gsync(DWs<double>& d, ModalBar* bar, int C
     return *drem(&d.xs[15], 0) != 0.0;
 }
 
-// Polarisation of one slot (a sample pair, or a complex sample on an envelope grid) of a node
-// times e_c, Kerr responses only, without the time window: the expressions of modal_node_kernel
+// Polarisation of one slot of a node times e_c, Kerr responses only, without the time window: a
+// sample pair of two components, or a complex envelope sample of one or two; the expressions of modal_node_kernel
 // and modal_kerr2_kernel. f holds the components of the node's field.
 __device__ __forceinline__ cpx<double> modal_kerr(const LunaInst& I, int npol, double kc, int n, cpx<double> fx,
                                                   cpx<double> fy, double ex, double ey) {
     if (I.kind == 0) {
-        if (npol == 1) return mk<double>(ex * (kc * (fx.x * fx.x * fx.x)), ex * (kc * (fx.y * fx.y * fx.y)));
         const double k0 = kc * (fx.x * fx.x + fy.x * fy.x), k1 = kc * (fx.y * fx.y + fy.y * fy.y);
         return mk<double>(ex * (k0 * fx.x) + ey * (k0 * fy.x), ex * (k1 * fx.y) + ey * (k1 * fy.y));
     }
@@ -548,6 +547,7 @@ modal_dist_kernel(const LunaInst* inst, const double2* A, ModalArgs a, double2* 
         const double w0 = l == 0 ? 1.0 : 0.0, wa = l == 0 ? a.wlow : 0.0, wb = l == 0 ? __ldg(wl) : 1.0;
         ModalState* ms = a.ms;
         double* part = (l & 1) ? ms->part1 : ms->part;
+        double e2 = 0, v2 = 0;
         for (int c = cl; c < nm; c += C) {
             for (int n = tid; n < Mb; n += T) {
                 cpx<double> x = mk<double>(0, 0);
@@ -556,7 +556,20 @@ modal_dist_kernel(const LunaInst* inst, const double2* A, ModalArgs a, double2* 
 #pragma unroll
                     for (int m = 0; m < 4; ++m)
                         if (m < nm) v[m] = Et[(size_t)m * Mt + base + n];
-#pragma unroll 2
+                    if (I.kind == 0 && np == 1) {  // the cubes of the field, the factors after the sum
+#pragma unroll 4
+                        for (int s = 0; s < ns; ++s) {
+                            const double* e = a.ems + (size_t)s * nm;
+                            cpx<double> f = mk<double>(0, 0);
+#pragma unroll
+                            for (int m = 0; m < 4; ++m)
+                                if (m < nm) f = f + scale(__ldg(e + m), v[m]);
+                            for (int m = 4; m < nm; ++m) f = f + scale(__ldg(e + m), Et[(size_t)m * Mt + base + n]);
+                            const double we = (l == 0 ? w0 : __ldg(wl + s)) * __ldg(e + c);
+                            x = x + scale(we, mk<double>(f.x * f.x * f.x, f.y * f.y * f.y));
+                        }
+                        x = scale(a.kerr * (sc * sc * sc), x);
+                    } else {
                     for (int s = 0; s < ns; ++s) {
                         const double* e = a.ems + (size_t)s * nm * np;
                         cpx<double> fx = mk<double>(0, 0), fy = fx;
@@ -574,6 +587,7 @@ modal_dist_kernel(const LunaInst* inst, const double2* A, ModalArgs a, double2* 
                         const double ey = np == 2 ? __ldg(e + c * np + 1) : 0.0;
                         const cpx<double> P = modal_kerr(I, np, a.kerr, base + n, scale(sc, fx), scale(sc, fy), __ldg(e + c * np), ey);
                         x = x + scale(l == 0 ? w0 : __ldg(wl + s), P);
+                    }
                     }
                     if (I.kind == 1) {
                         x = scale(__ldg(I.towin + base + n), x);
@@ -609,23 +623,26 @@ modal_dist_kernel(const LunaInst* inst, const double2* A, ModalArgs a, double2* 
                 d.xs[9] = sv;
             }
             dsync();
-            if (p == 0 && tid == 0) {
-                double e2 = 0, v2 = 0;
-                for (int j = 0; j < R; ++j) {
-                    const double* x = drem(d.xs, j);
-                    e2 += x[8];
-                    v2 += x[9];
+            if (tid < 32 && (C == 1 || p == 0)) {  // one cluster: every CTA adds the cluster's sums
+                double x = tid < R ? drem(d.xs, tid)[8] : 0.0, y = tid < R ? drem(d.xs, tid)[9] : 0.0;
+                x = warp_sum(x);
+                y = warp_sum(y);
+                e2 += x;
+                v2 += y;
+                if (C > 1 && tid == 0) {
+                    part[2 * c] = x;
+                    part[2 * c + 1] = y;
                 }
-                part[2 * c] = e2;
-                part[2 * c + 1] = v2;
             }
         }
-        if (!(ok = modal_gsync<R>(d, bar, C))) break;
+        if (C > 1 && !(ok = modal_gsync<R>(d, bar, C))) break;
         if (tid == 0) {  // every CTA adds the same sums in the same order: identical decisions
-            double e2 = 0, v2 = 0;
-            for (int m = 0; m < nm; ++m) {
-                e2 += __ldcg(part + 2 * m);
-                v2 += __ldcg(part + 2 * m + 1);
+            if (C > 1) {
+                e2 = v2 = 0;
+                for (int m = 0; m < nm; ++m) {
+                    e2 += __ldcg(part + 2 * m);
+                    v2 += __ldcg(part + 2 * m + 1);
+                }
             }
             const double err = sqrt(e2), val = sqrt(v2);
             s_done = err <= a.atol || err <= a.rtol * val || l >= a.lmax;
@@ -639,6 +656,7 @@ modal_dist_kernel(const LunaInst* inst, const double2* A, ModalArgs a, double2* 
     }
     if (!ok && tid == 0) atomicOr(flags, 1 << ST_WAIT_TIMEOUT);
     if (ok && dst) {
+        __syncthreads();
         for (int c = cl; c < nm; c += C)
             for (int k = p + R * tid; k < Nw; k += R * T) {
                 const size_t e = (size_t)c * Nw + k;
