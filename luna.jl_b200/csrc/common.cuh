@@ -92,4 +92,12 @@ enum {
     ST_WAIT_TIMEOUT = 5,  // a bounded device-side wait (tensor-core completion) ran out
 };
 
+// Programmatic dependent launches: a kernel of a chain is scheduled while its predecessor runs, does what
+// does not depend on it, and waits here for its end (and with it for every earlier one); the next
+// of the chain may then be scheduled. Both are without effect in a plain launch.
+__device__ __forceinline__ void pdl_sync() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
+}
+
 }  // namespace luna

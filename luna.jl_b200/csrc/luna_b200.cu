@@ -1855,18 +1855,43 @@ float bf16_val(uint16_t h) {
     return f;
 }
 
+// A launch that may be scheduled before the kernel ahead of it has ended: for kernels that open with
+// pdl_sync (chains of launches of a few microseconds).
+template <typename... P, typename... A>
+void launch_pdl(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);  // errors: cudaGetLastError of the caller
+}
+
 // Er = A Mi^T or Pk = Pw Mf^T along the radial index of the 2Nw x Nr real view: FP64
-// CUDA-core tiles for the plain path, 3xBF16 tensor-core products for the mixed path.
+// CUDA-core tiles for the plain path, 3xBF16 tensor-core products for the mixed path. FP64 takes
+// 64 x 64 tiles where they occupy most SMs (half of 148: above, the larger tile's fewer
+// shared-memory reads a product count), 32 x 32 below.
 int rad_qdht(luna_radial_plan* p, const void* X, bool fwd, void* Y, const RadState* st, int* flags, cudaStream_t s) {
     const int rows = 2 * p->Nw;
     if (p->precision == LUNA_PREC_FP64) {
-        dim3 g((rows + RG_BM - 1) / RG_BM, (p->Nr + RG_BN - 1) / RG_BN);
-        rad_gemm_f64<<<g, 256, 0, s>>>((const double*)X, rows, rows, fwd ? p->Mf : p->Mi, (double*)Y, p->Nr, st);
+        const int g64 = (rows + 63) / 64 * ((p->Nr + 63) / 64);
+        const double* Mx = fwd ? p->Mf : p->Mi;
+        if (g64 >= 74)
+            launch_pdl(rad_gemm_f64<64>, dim3((rows + 63) / 64, (p->Nr + 63) / 64), 256, 0, s, (const double*)X, rows, rows, Mx,
+                       (double*)Y, p->Nr, st);
+        else
+            launch_pdl(rad_gemm_f64<32>, dim3((rows + 31) / 32, (p->Nr + 31) / 32), 128, 0, s, (const double*)X, rows, rows, Mx,
+                       (double*)Y, p->Nr, st);
     } else {
         dim3 g((rows + TC_BM - 1) / TC_BM, p->Nr / RAD_TC_BN);
         const int* fin = st ? (const int*)((const char*)st + offsetof(RadState, finished)) : nullptr;
-        tc_gemm_3xbf16<RAD_TC_BN><<<g, TC_THREADS, tc_smem_bytes<RAD_TC_BN>(), s>>>(
-            (const float*)X, rows, rows, fwd ? p->Mf_t : p->Mi_t, (float*)Y, p->Nr, fin, flags);
+        launch_pdl(tc_gemm_3xbf16<RAD_TC_BN>, g, TC_THREADS, tc_smem_bytes<RAD_TC_BN>(), s, (const float*)X, rows, rows,
+                   fwd ? p->Mf_t : p->Mi_t, (float*)Y, p->Nr, fin, flags);
     }
     return LUNA_OK;
 }
@@ -1876,8 +1901,8 @@ int rad_qdht(luna_radial_plan* p, const void* X, bool fwd, void* Y, const RadSta
 template <typename Rl>
 int rad_transform(luna_radial_plan* p, const TwTab<Rl>& tw, RadState* st, int* flags, cudaStream_t s) {
     rad_qdht(p, p->A, false, p->B, st, flags, s);
-    rad_column_kernel<Rl><<<p->Nr, LUNA_BLOCK, p->smem, s>>>(p->d_col, (const cpx<Rl>*)p->B, (cpx<Rl>*)p->A, tw,
-                                                            p->smem, p->gscr, p->gstride, st, flags);
+    launch_pdl(rad_column_kernel<Rl>, dim3(p->Nr), LUNA_BLOCK, p->smem, s, p->d_col, (const cpx<Rl>*)p->B, (cpx<Rl>*)p->A, tw,
+               p->smem, p->gscr, p->gstride, st, flags);
     rad_qdht(p, p->A, true, p->B, st, flags, s);
     return LUNA_OK;
 }
@@ -1896,9 +1921,9 @@ int rad_rhs(luna_radial_plan* p, const double2* Ew, double2* nl, cudaStream_t s,
         a.outfac = p->ofz;
     }
     CK(cudaMemsetAsync(p->d_flags, 0, sizeof(int), s));
-    rad_stage_kernel<Rl, double><<<rad_grid(n), 256, 0, s>>>(a, -1, Ew, (cpx<Rl>*)p->A);
+    launch_pdl(rad_stage_kernel<Rl, double>, dim3(rad_grid(n)), 256, 0, s, a, -1, Ew, (cpx<Rl>*)p->A);
     rad_transform<Rl>(p, t, nullptr, p->d_flags, s);
-    rad_store_kernel<Rl, double><<<rad_grid(n), 256, 0, s>>>(a, -1, (const cpx<Rl>*)p->B, nl);
+    launch_pdl(rad_store_kernel<Rl, double>, dim3(rad_grid(n)), 256, 0, s, a, -1, (const cpx<Rl>*)p->B, (void*)nl);
     CK(cudaGetLastError());
     return LUNA_OK;
 }
@@ -2182,6 +2207,9 @@ int col_solve(PlanT* p, XF&& xform, const char* who, const double* linop, double
     cudaStream_t s = p->stream;
     RadArgs a{p->Nw, p->Nr, S.L, G.g ? S.ofz : p->outfac, S.e1, S.st};
     const int eg = rad_grid(n);
+    // FP64 without a gradient: a stage's store and the next stage's input in one launch
+    const bool fused = sizeof(Rl) == 8 && !G.g;
+    const int ng = (int)std::min<size_t>((n + 127) / 128, 148 * 16);
     int* flags_dev = (int*)((char*)S.st + offsetof(RadState, flags));
     const int* fin_dev = (const int*)((char*)S.st + offsetof(RadState, finished));
     rad_init_kernel<<<1, 32, 0, s>>>(S.st, S.opt, S.y, S.yn, S.d_k);
@@ -2195,19 +2223,19 @@ int col_solve(PlanT* p, XF&& xform, const char* who, const double* linop, double
     int chunk = 4;
     long long enq = 0;
     const long long cap = (o->max_steps > 0) ? o->max_steps : (long long)1 << 40;
+    rad_begin_kernel<<<1, 32, 0, s>>>(S.st, S.opt);
     while (true) {
         for (int q = 0; q < chunk; ++q) {
-            rad_begin_kernel<<<1, 32, 0, s>>>(S.st, S.opt);
             for (int sg = 0; sg < 6; ++sg) {
                 // L(z) and the output factor at this stage's node (make_prop!, RK45.jl:284-297)
                 if (G.g) rad_gradfill_kernel<<<eg, 256, 0, s>>>(a, G, sg, 0.0, S.L, S.ofz);
-                rad_stage_kernel<Rl, Kt><<<eg, 256, 0, s>>>(a, sg, nullptr, (cpx<Rl>*)p->A);
+                if (sg == 0 || !fused) launch_pdl(rad_stage_kernel<Rl, Kt>, dim3(eg), 256, 0, s, a, sg, (const double2*)nullptr, (cpx<Rl>*)p->A);
                 xform(t, S.st, flags_dev, s);
-                rad_store_kernel<Rl, Kt><<<eg, 256, 0, s>>>(a, sg, (const cpx<Rl>*)p->B, nullptr);
+                if (sg == 5 || !fused) launch_pdl(rad_store_kernel<Rl, Kt>, dim3(eg), 256, 0, s, a, sg, (const cpx<Rl>*)p->B, (void*)nullptr);
+                else launch_pdl(rad_next_kernel, dim3(ng), 128, 0, s, a, sg, (const cpx<double>*)p->B, (cpx<double>*)p->A);
             }
-            rad_combine_kernel<Kt><<<nblk, 256, 0, s>>>(a, S.partial);
-            rad_control_kernel<<<1, 256, 0, s>>>(S.st, S.opt, S.partial, nblk);
-            rad_post_kernel<Rl, Kt><<<p->Nr, LUNA_BLOCK, p->smem, s>>>(a, p->d_col, S.opt, t, p->smem, p->gscr, p->gstride, G);
+            launch_pdl(rad_combine_kernel<Kt>, dim3(nblk), 256, 0, s, a, S.partial, S.opt);
+            launch_pdl(rad_post_kernel<Rl, Kt>, dim3(p->Nr), LUNA_BLOCK, p->smem, s, a, p->d_col, S.opt, t, p->smem, p->gscr, p->gstride, G);
         }
         CK(cudaGetLastError());
         enq += chunk;

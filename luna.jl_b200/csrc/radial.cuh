@@ -33,6 +33,7 @@ struct RadState {
     int nsaved;          // save points taken so far
     int save_lo, save_hi;  // save points taken by the current accepted step
     int flags;           // status bits raised by the column kernels
+    unsigned ticket[2];  // blocks of the combining and of the closing kernel that have finished
 };
 
 struct RadArgs {
@@ -133,6 +134,7 @@ __global__ void __launch_bounds__(256) rad_gradfill_kernel(RadArgs a, RadGrad G,
 // kernel, one element per thread); s < 0: A = src (a plain right-hand side evaluation).
 template <typename Rl, typename Kt>
 __global__ void __launch_bounds__(256) rad_stage_kernel(RadArgs a, int s, const double2* src, cpx<Rl>* A) {
+    pdl_sync();
     const RadState* st = a.st;
     if (st && st->finished) return;
     const size_t n = (size_t)a.Nw * a.Nr;
@@ -174,6 +176,7 @@ __global__ void __launch_bounds__(256) rad_stage_kernel(RadArgs a, int s, const 
 // output of a plain right-hand side evaluation).
 template <typename Rl, typename Kt>
 __global__ void __launch_bounds__(256) rad_store_kernel(RadArgs a, int s, const cpx<Rl>* Pk, void* dst) {
+    pdl_sync();
     const RadState* st = a.st;
     if (st && st->finished) return;
     const size_t n = (size_t)a.Nw * a.Nr;
@@ -194,69 +197,117 @@ __global__ void __launch_bounds__(256) rad_store_kernel(RadArgs a, int s, const 
     }
 }
 
+// rad_store_kernel of stage s and rad_stage_kernel of stage s + 1 (s = 0..4) for the same element in one
+// launch (FP64; with a gas fill gradient L changes in between). Two stages at one node share their
+// exponential. 6.3 us as two launches at 257 x 64, bound by the latency of the
+// exponential, sine and cosine of one element a thread: 128 threads a block spread it over the SMs.
+__global__ void __launch_bounds__(128) rad_next_kernel(RadArgs a, int s, const cpx<double>* Pk, cpx<double>* A) {
+    pdl_sync();
+    const RadState* st = a.st;
+    if (st->finished) return;
+    const size_t n = (size_t)a.Nw * a.Nr;
+    const cpx<double>* of = reinterpret_cast<const cpx<double>*>(a.outfac);
+    const cpx<double>* L = reinterpret_cast<const cpx<double>*>(a.L);
+    const cpx<double>* y = reinterpret_cast<const cpx<double>*>(st->y);
+    cpx<double>* e1 = reinterpret_cast<cpx<double>*>(a.e1);
+    const double t0 = st->c.t, dt = st->c.dt;
+    const double d0 = __dsub_rn(__dadd_rn(t0, __dmul_rn(c_nodes[s], dt)), t0);
+    const double d1 = __dsub_rn(__dadd_rn(t0, __dmul_rn(c_nodes[s + 1], dt)), t0);
+    cpx<double>* k[7];
+#pragma unroll
+    for (int j = 0; j < 7; ++j) k[j] = reinterpret_cast<cpx<double>*>(st->c.k[j]);
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const cpx<double> Li = L[i];
+        cpx<double> acc = y[i];
+        for (int j = 0; j <= s; ++j) {
+            const double bj = c_B[s + 1][j];
+            if (bj != 0) acc = acc + scale(dt * bj, k[j][i]);
+        }
+        const cpx<double> f0 = expLd<double>(Li, d0);
+        const cpx<double> f1 = d1 == d0 ? f0 : expLd<double>(Li, d1);
+        const cpx<double> v = (Pk[i] * of[i]) * inv_fac<double>(f0);
+        k[s + 1][i] = v;
+        if (s + 1 == 4) e1[i] = f1;
+        acc = acc + scale(dt * c_B[s + 1][s + 1], v);
+        A[i] = f1 * acc;
+    }
+}
+
 // ------------------------------------------------------------------ QDHT products (FP64)
 // C[r, n] = sum_m A[r + m*lda] * B[n*K + m] for r < rows, n < N (= K = Nr): the QDHT
 // matrix B (row-major Nr x Nr) applied along the radial index of the column-major
-// 2Nw x Nr real view of a complex Nw x Nr array. 64 x 64 output tile per CTA, 16-deep
-// K slices staged in shared memory, 4 x 4 outputs per thread.
-#define RG_BM 64
-#define RG_BN 64
-#define RG_BK 16
-__global__ void __launch_bounds__(256) rad_gemm_f64(const double* __restrict__ A, int lda, int rows,
-                                                    const double* __restrict__ B, double* __restrict__ C, int K,
-                                                    const RadState* st) {
-    if (st && st->finished) return;
-    __shared__ double As[2][RG_BK][RG_BM];
-    __shared__ double Bs[2][RG_BK][RG_BN + 1];
+// 2Nw x Nr real view of a complex Nw x Nr array. T x T outputs a CTA (T = 64: 256 threads with
+// 4 x 4 each; T = 32: 128 with 4 x 2), K slices of KB streamed by cp.async into a ring of four. Bound by the
+// latency of its few slices at small Nr (one slice at a time from registers, 64 x 64 tiles:
+// 6 us at 514 x 64 x 64 on 9 CTAs) and by FP64 and shared-memory rates at large ones. The sum over
+// m runs in order in either tile.
+template <int T>
+__global__ void __launch_bounds__(T == 64 ? 256 : 128)
+rad_gemm_f64(const double* __restrict__ A, int lda, int rows, const double* __restrict__ B, double* __restrict__ C,
+             int K, const RadState* st) {
+    constexpr int KB = T == 64 ? 8 : 16, ST = 4, NT = T == 64 ? 256 : 128, TX = T / 4, TN = T * TX / NT;
+    __shared__ double As[ST][KB][T];
+    __shared__ double Bs[ST][KB][T + 1];
     const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;
-    const int r0 = blockIdx.x * RG_BM, n0 = blockIdx.y * RG_BN;
-    double acc[4][4];
+    const int tx = tid % TX, ty = tid / TX;
+    const int r0 = blockIdx.x * T, n0 = blockIdx.y * T;
+    pdl_sync();
+    if (st && st->finished) return;
+    double acc[4][TN];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
-    // loaders: A slice 16 x 64 (4 per thread, coalesced along r); B slice 64 x 16 (4 per
-    // thread, coalesced along m)
-    auto load = [&](int kb, int buf) {
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0.0;
+    const int ns = (K + KB - 1) / KB;
+    // A slice KB x T coalesced along r, B slice T x KB along m; zero-filled past the edges
+    auto load = [&](int sl) {
+        if (sl < ns) {
+            const int buf = sl % ST, kb = sl * KB;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int e = tid + 256 * q;
-            const int kk = e >> 6, rr = e & 63;
-            const int r = r0 + rr, m = kb + kk;
-            As[buf][kk][rr] = (r < rows && m < K) ? A[(size_t)m * lda + r] : 0.0;
-            const int nn = e >> 4, mk = e & 15;
-            const int nB = n0 + nn, mB = kb + mk;
-            Bs[buf][mk][nn] = (nB < K && mB < K) ? B[(size_t)nB * K + mB] : 0.0;
+            for (int q = 0; q < KB * T / NT; ++q) {
+                const int e = tid + NT * q;
+                const int kk = e / T, rr = e % T, r = r0 + rr, m = kb + kk;
+                const bool oa = r < rows && m < K;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((unsigned)__cvta_generic_to_shared(&As[buf][kk][rr])),
+                             "l"(oa ? A + (size_t)m * lda + r : A), "r"(oa ? 8 : 0)
+                             : "memory");
+                const int nn = e / KB, mk = e % KB, nB = n0 + nn, mB = kb + mk;
+                const bool ob = nB < K && mB < K;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((unsigned)__cvta_generic_to_shared(&Bs[buf][mk][nn])),
+                             "l"(ob ? B + (size_t)nB * K + mB : B), "r"(ob ? 8 : 0)
+                             : "memory");
+            }
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    load(0, 0);
-    __syncthreads();
-    int buf = 0;
-    for (int kb = 0; kb < K; kb += RG_BK) {
-        if (kb + RG_BK < K) load(kb + RG_BK, buf ^ 1);
 #pragma unroll
-        for (int kk = 0; kk < RG_BK; ++kk) {
-            double av[4], bv[4];
+    for (int q = 0; q < ST - 1; ++q) load(q);
+    for (int sl = 0; sl < ns; ++sl) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
+        __syncthreads();  // slice sl has landed, and every thread is done with slice sl - 1
+        load(sl + ST - 1);
+        const int buf = sl % ST;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) av[i] = As[buf][kk][tx + 16 * i];
+        for (int kk = 0; kk < KB; ++kk) {
+            double av[4], bv[TN];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) bv[j] = Bs[buf][kk][ty + 16 * j];
+            for (int i = 0; i < 4; ++i) av[i] = As[buf][kk][tx + TX * i];
+#pragma unroll
+            for (int j = 0; j < TN; ++j) bv[j] = Bs[buf][kk][ty + (T / TN) * j];
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fma(av[i], bv[j], acc[i][j]);
+                for (int j = 0; j < TN; ++j) acc[i][j] = fma(av[i], bv[j], acc[i][j]);
         }
-        __syncthreads();
-        buf ^= 1;
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const int r = r0 + tx + 16 * i;
+        const int r = r0 + tx + TX * i;
         if (r >= rows) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + ty + 16 * j;
+        for (int j = 0; j < TN; ++j) {
+            const int n = n0 + ty + (T / TN) * j;
             if (n < K) C[(size_t)n * lda + r] = acc[i][j];
         }
     }
@@ -277,7 +328,6 @@ __global__ void __launch_bounds__(LUNA_BLOCK, sizeof(Rl) == 4 ? 2 : 1)
 rad_column_kernel(const LunaInst* inst, const cpx<Rl>* Er, cpx<Rl>* Pw, TwTab<Rl> tw, int smem_bytes,
                   char* gscr, size_t gstride, RadState* st, int* flags) {
     char* const smem = dsm;
-    if (st && st->finished) return;
     __shared__ LunaInst sI;
     tws_fill(tw);
     const LunaInst& I = local_inst<Rl>(inst, &sI);
@@ -285,6 +335,8 @@ rad_column_kernel(const LunaInst* inst, const cpx<Rl>* Er, cpx<Rl>* Pw, TwTab<Rl
     Ws<Rl> w;
     plan_ws<Rl>(I, smem, smem_bytes, w, tw, gscr ? gscr + (size_t)c * gstride : nullptr);
     if (threadIdx.x == 0) *w.flag = 0;
+    pdl_sync();
+    if (st && st->finished) return;
     __syncthreads();
     const cpx<Rl>* E = Er + (size_t)c * I.Nw;
     cpx<Rl>* o = Pw + (size_t)c * I.Nw;
@@ -313,12 +365,13 @@ __global__ void rad_init_kernel(RadState* st, LunaInst* opt, double2* y, double2
     st->nsaved = 0;
     st->save_lo = st->save_hi = 0;
     st->flags = 0;
+    st->ticket[0] = st->ticket[1] = 0;
     opt->accepted = opt->rejected = 0;
 }
 
-// Loop head of RK45.solve / evaluate! (RK45.jl:43-78, 209-223).
-__global__ void rad_begin_kernel(RadState* st, const LunaInst* opt) {
-    if (threadIdx.x != 0 || blockIdx.x != 0 || st->finished) return;
+// Loop head of RK45.solve / evaluate! (RK45.jl:43-78, 209-223), one thread: before the first step
+// in its own launch, then by the last block of rad_post_kernel.
+__device__ __forceinline__ void rad_begin(RadState* st, const LunaInst* opt) {
     Ctl& c = st->c;
     if (!(c.tn <= opt->zmax) || c.done) {
         st->finished = 1;
@@ -333,11 +386,32 @@ __global__ void rad_begin_kernel(RadState* st, const LunaInst* opt) {
     c.dt = c.dtn;
     c.t = c.tn;
 }
+__global__ void rad_begin_kernel(RadState* st, const LunaInst* opt) {
+    pdl_sync();
+    if (threadIdx.x == 0 && blockIdx.x == 0 && !st->finished) rad_begin(st, opt);
+}
+
+// True in the block that finishes last (its threads see the others' writes).
+__device__ __forceinline__ bool rad_last_block(unsigned* ticket) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        if (last) *ticket = 0;
+        __threadfence();
+    }
+    __syncthreads();
+    return last;
+}
+
+__device__ void rad_control(RadState* st, LunaInst* opt, const double* partial, int nblocks);
 
 // yn = y + dt sum b5_j k_j and the three sums of the weak norm, per block (fixed
 // partition, so the reduction order does not change from run to run).
 template <typename Kt>
-__global__ void __launch_bounds__(256) rad_combine_kernel(RadArgs a, double* partial) {
+__global__ void __launch_bounds__(256) rad_combine_kernel(RadArgs a, double* partial, LunaInst* opt) {
+    pdl_sync();
     const RadState* st = a.st;
     if (st->finished) return;
     __shared__ double red[3 * 8];
@@ -390,20 +464,20 @@ __global__ void __launch_bounds__(256) rad_combine_kernel(RadArgs a, double* par
         partial[3 * blockIdx.x + 1] = a1;
         partial[3 * blockIdx.x + 2] = a2;
     }
+    if (rad_last_block(&a.st->ticket[0])) rad_control(a.st, opt, partial, gridDim.x);
 }
 
 // Weak norm, PI controller and bookkeeping (the same code as the fused solver), FSAL
-// rotation and the save points the accepted step covers. One CTA of 256 threads: thread t
+// rotation and the save points the accepted step covers, by the last block of
+// rad_combine_kernel (a launch of its own was 3 us a step). 256 threads: thread t
 // sums the partials t, t+256, ... in order, then a fixed-order tree (deterministic).
-__global__ void __launch_bounds__(256) rad_control_kernel(RadState* st, LunaInst* opt, const double* partial,
-                                                          int nblocks) {
-    if (st->finished) return;
+__device__ void rad_control(RadState* st, LunaInst* opt, const double* partial, int nblocks) {
     __shared__ double red[3][256];
     double sy = 0, syn = 0, se = 0;
     for (int b = threadIdx.x; b < nblocks; b += 256) {
-        sy += partial[3 * b];
-        syn += partial[3 * b + 1];
-        se += partial[3 * b + 2];
+        sy += __ldcg(partial + 3 * b);
+        syn += __ldcg(partial + 3 * b + 1);
+        se += __ldcg(partial + 3 * b + 2);
     }
     red[0][threadIdx.x] = sy;
     red[1][threadIdx.x] = syn;
@@ -452,21 +526,23 @@ __global__ void __launch_bounds__(LUNA_BLOCK, 1)
 rad_post_kernel(RadArgs a, const LunaInst* inst, const LunaInst* opt, TwTab<Rl> tw, int smem_bytes, char* gscr,
                 size_t gstride, RadGrad G) {
     char* const smem = dsm;
-    const RadState* st = a.st;
-    if (st->finished) return;
+    RadState* st = a.st;
     __shared__ LunaInst sI;
     tws_fill(tw);
     const LunaInst& I = local_inst<Rl>(inst, &sI);
     const int c = blockIdx.x, Nw = a.Nw;
     const size_t off = (size_t)c * Nw;
+    Ws<Rl> w;
+    plan_ws<Rl>(I, smem, smem_bytes, w, tw, gscr ? gscr + (size_t)c * gstride : nullptr);
+    pdl_sync();
+    if (st->finished) return;
     double2* y = st->y + off;
     double2* yn = st->yn + off;
     if (!st->c.ok) {
         for (int i = threadIdx.x; i < Nw; i += LUNA_BLOCK) yn[i] = y[i];
+        if (rad_last_block(&st->ticket[1]) && threadIdx.x == 0) rad_begin(st, opt);
         return;
     }
-    Ws<Rl> w;
-    plan_ws<Rl>(I, smem, smem_bytes, w, tw, gscr ? gscr + (size_t)c * gstride : nullptr);
     stepfun_filter<Rl>(I, w, yn, a.e1 + off);
     void* kc[7];
 #pragma unroll
@@ -490,6 +566,7 @@ rad_post_kernel(RadArgs a, const LunaInst* inst, const LunaInst* opt, TwTab<Rl> 
         interpolate_row<Rl, Kt>(Nw, a.L + off, st->c, opt->zsave[si], kc, y, yn,
                                 opt->saves + (size_t)si * Nw * a.Nr + off);
     }
+    if (rad_last_block(&st->ticket[1]) && threadIdx.x == 0) rad_begin(st, opt);
 }
 
 }  // namespace luna

@@ -154,6 +154,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 tc_gemm_3xbf16(const float* __restrict__ A, int lda, int rows, const __nv_bfloat16* __restrict__ Bt,
                float* __restrict__ C, int K, const int* finished, int* flags) {
     static_assert(BN % 32 == 0 && BN >= 32 && BN <= 256, "BN must be a multiple of 32 in 32..256");
+    pdl_sync();
     if (finished && *finished) return;
     extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
     __shared__ __align__(8) uint64_t mbar[4];  // 0, 1: MMAs of stage s done; 2, 3: B of stage s landed
