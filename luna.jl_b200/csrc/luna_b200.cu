@@ -417,6 +417,14 @@ grad_linop_kernel(LunaInst I, double z, double2* L, double2* of) {
     grad_fill_to(I, bc, z, true, L, of);
 }
 
+// LunaResp::spk from the tables of the ionisation spline
+__global__ void pack_nodes_kernel(const double* x, const double* y, const double* D, int n, double2* out) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= n) return;
+    out[2 * (size_t)j] = make_double2(x[j], y[j]);
+    out[2 * (size_t)j + 1] = make_double2(D[j], 0.0);
+}
+
 // Raman response spectrum at plan creation (Raman.jl:256-262, Nonlinear.jl:306-307):
 // h(t) = w(t) * sum_c hpre_c(t) exp(-t/tau2_c) on the first half of a 2*No grid,
 // H[k] = rfft(hscale * h)[k], k = 0..No, computed in FP64. The response is normalised by
@@ -1033,16 +1041,13 @@ int luna_b200_plan_create(const luna_grid_desc* g, const luna_resp_desc* resps, 
                     UP(d.spl_y, d.spl_n, &r.sy);
                     UP(d.spl_D, d.spl_n, &r.sD);
                     if (precision == LUNA_PREC_FP64) {
-                        std::vector<double> pk(4 * (size_t)d.spl_n);
-                        for (int j = 0; j < d.spl_n; ++j) {
-                            pk[4 * (size_t)j] = d.spl_x[j];
-                            pk[4 * (size_t)j + 1] = d.spl_y[j];
-                            pk[4 * (size_t)j + 2] = d.spl_D[j];
-                            pk[4 * (size_t)j + 3] = 0.0;
-                        }
-                        const double* t = nullptr;
-                        UP(pk.data(), pk.size(), &t);
-                        r.spk = reinterpret_cast<const double2*>(t);
+                        double2* t = nullptr;  // packed on the device: no second upload
+                        if (dalloc(p->allocs, &t, 2 * sizeof(double2) * (size_t)d.spl_n)) { free_all(p->allocs); delete p; return LUNA_ERR_CUDA; }
+                        pack_nodes_kernel<<<(d.spl_n + 255) / 256, 256>>>(r.sx, r.sy, r.sD, d.spl_n, t);
+                        cudaError_t e = cudaGetLastError();
+                        if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+                        if (e != cudaSuccess) { free_all(p->allocs); delete p; return fail(LUNA_ERR_CUDA, std::string("pack_nodes_kernel: ") + cudaGetErrorString(e)); }
+                        r.spk = t;
                         r.sn = d.spl_n;
                         r.Emin = d.spl_x[0];
                         r.Emax = d.spl_x[d.spl_n - 1];
