@@ -132,7 +132,8 @@ typedef struct {
     long long stats_cap;                       /* rows of per-step statistics; 0: off       */
     int dist_min_no;                           /* batches: instances with at least this many
                                                   oversampled samples run on a cluster of CTAs
-                                                  each (in the batch's precision); 0: 16384  */
+                                                  each (in the batch's precision); 0: 4096 in
+                                                  full precision, 16384 in mixed             */
 } luna_solve_opts;
 
 /* Per-step statistics (Stats.default, Stats.jl:495-532, for a mode-averaged field-resolved

@@ -24,11 +24,6 @@ extern "C" {
  * (stride N); outputs [B x N] (stride B*N): Y BF16, Zout BF16, Yf FP32, each may be NULL. */
 int luna_sg_linear_fwd(const void* X, long long sX, const void* W, const float* b, int B, int K, int N, int act,
                        void* Y, void* Zout, float* Yf, int members, int* err, void* stream);
-/* The last layer with its ensemble statistics: luna_sg_linear_fwd (act 0, FP32 outputs) followed
- * by luna_sg_ensemble, without storing the members' outputs. mean [B x N] must be 16-byte
- * aligned; members share X when sX is 0. */
-int luna_sg_linear_ensemble(const void* X, long long sX, const void* W, const float* b, int B, int K, int N, int nspec,
-                            float* mean, float* spread, int members, int* err, void* stream);
 /* Backward through the layer's input: dXpre = (dZ W) * silu'(Zprev), [B x K] BF16. */
 int luna_sg_linear_bwd_data(const void* dZ, const void* W, const void* Zprev, int B, int K, int N, void* dXpre,
                             int members, int* err, void* stream);

@@ -3,7 +3,7 @@ scans run one ``prop_capillary`` after another, Scans.jl:275-353).
 
 For every grid class of a batch (oversampled length No and whether a Raman response is
 present) and the batch's precision it measures the device time of one RK step on one CTA,
-on an 8-CTA cluster and (for the 32768-point grids) on a 16-CTA cluster (a batch of one
+on an 8-CTA cluster and (for the longest grids) on a 16-CTA cluster (a batch of one
 representative instance, the difference of two step budgets, CUDA events), once per device,
 and caches the table in a JSON file (``$LUNA_B200_TUNE_CACHE``, default
 ``~/.cache/luna_b200/tune.json``). An instance's
@@ -93,7 +93,8 @@ def measure(probs, precision, steps=(20, 80), refresh=False, log=None, tries=8):
                 continue
             cl, on = _step_ms(p, precision, 0, steps, shape=2)
             row = {"single": single, "cluster": cl if on else None, "cluster16": None}
-            if on and p.grid.No >= 32768:  # 16 CTAs need 1024 sample pairs each
+            # 16 CTAs need 512 sample pairs each in full precision, 1024 in mixed
+            if on and p.grid.No // 32 >= (512 if precision == _lib.PREC_FP64 else 1024):
                 c16, on16 = _step_ms(p, precision, 0, steps, shape=3)
                 row["cluster16"] = c16 if on16 else None
             break

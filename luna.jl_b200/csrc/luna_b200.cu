@@ -387,7 +387,8 @@ rhs_kernel(LunaInst* inst, const double2* Ew, double2* nl, TwTab<Rl> tw, int sme
 
 // The same on a cluster of R CTAs in FP64 (constant fill, no analytic-signal responses), the
 // right-hand side of the distributed solver. Bound by latency as on one CTA, but every loop over
-// bins and samples is 1/R as long and the sub-transforms are log2 R levels shorter.
+// bins and samples is 1/R as long and the sub-transforms are log2 R levels shorter: He, No = 4096,
+// 31 us on one CTA, 24.6 on 4; H2 with Raman, No = 32768, 518 and 61.5 us on 16.
 template <int R>
 __global__ void __launch_bounds__(LUNA_BLOCK, 1)
 rhs_kernel_dist(const LunaInst* inst, const double2* Ew, double2* nl, TwTab<double> tw, int* status) {
@@ -759,12 +760,11 @@ bool dist_fits(const LunaInst& I, int R) {
 }
 
 // Which instances of a batch run distributed, from per-instance work estimates (single-CTA time in
-// any unit). Mixed precision: the eligible ones whose estimate is at least the mean load of an SM
-// (total / SMs), i.e. the long poles of the batch, on clusters of DIST_R, from four times that on
-// DIST_R_BIG. FP64: the number k of instances, longest first, for which the larger of the mean
-// SM load and the longest single run is smallest, a cluster of DIST_R taking 1/3 of the time of one CTA
-// (measured 2.5-4) and so 8/3 of its SM time; all of them on DIST_R_BIG when that many fit at
-// once (a cluster of 16 takes about 3/4 of the time of one of 8, i.e. more SM time). Shapes set
+// any unit): the eligible ones whose estimate is at least the mean load of an SM (total / SMs), i.e.
+// the long poles of the batch, on clusters of DIST_R, from four times that on DIST_R_BIG. On a cluster
+// of 8 an FP64 instance takes 1/2 (No = 8192) to 1/4.6 (32768 with Raman) of its time on one CTA, on
+// 16 3/4 of that. 96 FP64 instances: 97 ms with this rule, 405 ms on single CTAs, 115 ms all on
+// clusters; 24: 48, 299 and 66 ms; 48: 66, 300 and 68 ms; 192: 181, 511 and 214 ms. Shapes set
 // per instance come first. Every SM that can hold a cluster starts as one (longest instances
 // first); the single-CTA instances fill the SMs left over and the clusters once their list is
 // empty. All lists in priority order.
@@ -776,40 +776,11 @@ int dist_partition(luna_batch* b, const double* pr) {
     auto shape = [&](int i) { return b->shape.empty() ? 0 : b->shape[i]; };
     double W = 0;
     for (int i = 0; i < n; ++i) W += pr[i];
-    if (b->precision == LUNA_PREC_FP64) {
-        std::vector<int> ord(b->elig);
-        std::stable_sort(ord.begin(), ord.end(), [&](int a, int c) { return pr[a] > pr[c]; });
-        std::vector<char> el(n, 0);
-        for (int i : ord) el[i] = 1;
-        double rest = 0;  // longest instance that cannot be distributed
-        for (int i = 0; i < n; ++i)
-            if (!el[i]) rest = std::max(rest, pr[i]);
-        double best = 0, load = W;
-        size_t k = 0;
-        for (size_t j = 0; j <= ord.size(); ++j) {
-            if (j > 0) load += (8.0 / 3.0 - 1.0) * pr[ord[j - 1]];
-            const double longest = std::max(std::max(rest, j < ord.size() ? pr[ord[j]] : 0.0), j > 0 ? pr[ord[0]] / 3.0 : 0.0);
-            const double t = std::max(load / std::max(1, b->nsm), longest);
-            if (j == 0 || t < best) {
-                best = t;
-                k = j;
-            }
-        }
-        for (size_t j = 0; j < k; ++j)
-            if (shape(ord[j]) == 0) isd[ord[j]] = 1;
-        for (int i : ord)
-            if (shape(i) >= 2) isd[i] = 1;
-        int nd = 0;
-        for (int i = 0; i < n; ++i) nd += isd[i];
-        for (int i = 0; i < n; ++i)
-            if (isd[i] && big[i] && (shape(i) == 3 || (shape(i) == 0 && nd <= b->ncl16_max))) isd[i] = 2;
-    } else {
-        const double thr = W / std::max(1, b->nsm);
-        for (int i : b->elig) {
-            const int sh = shape(i);
-            isd[i] = sh == 2 || sh == 3 || (sh == 0 && pr[i] >= thr);
-            if (isd[i] && big[i] && (sh == 3 || (sh == 0 && pr[i] >= 4.0 * thr))) isd[i] = 2;
-        }
+    const double thr = W / std::max(1, b->nsm);
+    for (int i : b->elig) {
+        const int sh = shape(i);
+        isd[i] = sh == 2 || sh == 3 || (sh == 0 && pr[i] >= thr);
+        if (isd[i] && big[i] && (sh == 3 || (sh == 0 && pr[i] >= 4.0 * thr))) isd[i] = 2;
     }
     b->dist.clear();
     b->dist16.clear();
@@ -2386,7 +2357,7 @@ int modal_dist(luna_modal_plan* p, const double2* src, double2* dst, const TwTab
 
 // Clusters of a plan: full precision, time buffers that give each CTA of a cluster 512
 // samples, and not the two-component plasma (its scans run on one CTA a node). As many clusters as
-// modes (Kerr alone: 33 us at No = 16384 with one mode, 330 us with the kernels of one CTA) or as nodes of
+// modes (Kerr alone: 72 us at No = 16384 with one mode, 332 us with the kernels of one CTA) or as nodes of
 // the third refinement, if that many are resident together.
 template <int R>
 bool modal_dist_setup(luna_modal_plan* p) {

@@ -424,8 +424,8 @@ modal_level_kernel(const LunaInst* inst, ModalArgs a, int l, cpx<Rl>* B, TwTab<R
 // time samples together, as a distributed right-hand side does (dist.cuh). Time samples are in natural
 // order, CTA q holding the block q. The kernels above run one CTA a mode, 17 to 19 launches of which
 // those after convergence do nothing: at No = 16384 with one mode and 15 nodes 25 us for the field,
-// 31 us for each level's nodes and 56 to 100 us for its integral. Bound by the chain of one transform
-// per level.
+// 31 us for each level's nodes and 56 to 100 us for its integral, 332 us in all; 72 us here. Bound by the
+// chain of one transform per level (16 k cycles each) and the exchange of its L2 sums.
 //
 // elem (Kerr responses alone): the integrand is local in time, so each level's sum over its nodes
 // is evaluated in registers from the mode fields, without G; nothing but the convergence

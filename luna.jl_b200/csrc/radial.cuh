@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(256) rad_store_kernel(RadArgs a, int s, const 
 
 // rad_store_kernel of stage s and rad_stage_kernel of stage s + 1 (s = 0..4) for the same element in one
 // launch (FP64; with a gas fill gradient L changes in between). Two stages at one node share their
-// exponential. 6.3 us as two launches at 257 x 64, bound by the latency of the
+// exponential. 11 us as two launches at 257 x 64 (profiler's clock), bound by the latency of the
 // exponential, sine and cosine of one element a thread: 128 threads a block spread it over the SMs.
 __global__ void __launch_bounds__(128) rad_next_kernel(RadArgs a, int s, const cpx<double>* Pk, cpx<double>* A) {
     pdl_sync();
@@ -238,8 +238,9 @@ __global__ void __launch_bounds__(128) rad_next_kernel(RadArgs a, int s, const c
 // matrix B (row-major Nr x Nr) applied along the radial index of the column-major
 // 2Nw x Nr real view of a complex Nw x Nr array. T x T outputs a CTA (T = 64: 256 threads with
 // 4 x 4 each; T = 32: 128 with 4 x 2), K slices of KB streamed by cp.async into a ring of four. Bound by the
-// latency of its few slices at small Nr (one slice at a time from registers, 64 x 64 tiles:
-// 6 us at 514 x 64 x 64 on 9 CTAs) and by FP64 and shared-memory rates at large ones. The sum over
+// latency of its few slices at small Nr (one slice at a time, 64 x 64 tiles: 10 us at
+// 514 x 64 x 64 on 9 CTAs under the profiler's clock; with the fused stages and dependent launches a
+// step of that size went from 0.33 to 0.19 ms) and by FP64 and shared-memory rates at large ones. The sum over
 // m runs in order in either tile.
 template <int T>
 __global__ void __launch_bounds__(T == 64 ? 256 : 128)
