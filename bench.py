@@ -1055,7 +1055,7 @@ def main():
                 v_sub, v_scan, rows = plain_fp64_measured(inst, probs, dur64, [x.status for x in st64])
                 plain = {"value": v_scan, "unit": "sims/hour", "subset_value": v_sub,
                          "method": ("plain FP64 drop-in measured: one single-instance FP64 solve after another "
-                                    f"(device time; clusters of 16 CTAs for No = 32768, of 8 for No = 16384) for {len(rows)} instances, "
+                                    f"(device time; clusters of 16 CTAs from No = 16384, of 8 for No = 8192) for {len(rows)} instances, "
                                     "8 quantiles of the single-CTA FP64 batch time in each of the two strata; value = "
                                     "the scan's sims/hour with each stratum's per-instance batch times scaled by its "
                                     "subset's measured/batch ratio, subset_value = the subset's own"),

@@ -630,7 +630,7 @@ namespace {
 // (or when an allocation fails). A block is given back after the device has finished all
 // work, cleared like a fresh one, so the next owner may use it on any stream and thread.
 struct DevPool {
-    static constexpr size_t POOL_KEEP = (size_t)256 << 20, POOL_BLOCK = (size_t)64 << 20;
+    static constexpr size_t POOL_KEEP = (size_t)64 << 20, POOL_BLOCK = (size_t)16 << 20;
     struct Block {
         size_t size;
         int dev;
