@@ -21,7 +21,9 @@ extern "C" {
 
 /* Linear layer forward: Z = X W^T + b, Y = act(Z) (act 1: SiLU, 0: identity). X [B x K]
  * BF16 (member stride sX, 0 to share one input), W [N x K] BF16 (stride N*K), b [N] FP32
- * (stride N); outputs [B x N] (stride B*N): Y BF16, Zout BF16, Yf FP32, each may be NULL. */
+ * (stride N); outputs [B x N] (stride B*N): Y BF16, Zout BF16, Yf FP32, each may be NULL.
+ * Here and in the backward products outputs and Zprev are 16-byte aligned (else
+ * LUNA_ERR_BAD_ARG, nothing is launched); b and db need the 4 bytes of an FP32 value. */
 int luna_sg_linear_fwd(const void* X, long long sX, const void* W, const float* b, int B, int K, int N, int act,
                        void* Y, void* Zout, float* Yf, int members, int* err, void* stream);
 /* Backward through the layer's input: dXpre = (dZ W) * silu'(Zprev), [B x K] BF16. */

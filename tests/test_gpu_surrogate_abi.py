@@ -1,0 +1,74 @@
+"""The surrogate library's C entry points on what their header allows beyond the package's own calls.
+Where the same operations run, results are equal; what is refused is refused before a launch."""
+import ctypes
+
+import luna_b200_loader  # registers the luna.jl_b200 package
+
+luna_b200_loader.load()
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _sg():
+    torch = pytest.importorskip("torch")
+    from luna_b200 import surrogate as S
+    return torch, S.load(), (lambda t: ctypes.c_void_p(t.data_ptr())), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+def _layer(torch, members, B, K, N, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    bf = torch.bfloat16
+    return dict(X=torch.randn(members, B, K, device="cuda", generator=g).to(bf),
+                W=(torch.randn(members, N, K, device="cuda", generator=g) / K ** 0.5).to(bf),
+                b=torch.randn(members, N, device="cuda", generator=g),
+                dZ=torch.randn(members, B, N, device="cuda", generator=g).to(bf),
+                Zp=torch.randn(members, B, K, device="cuda", generator=g).to(bf),
+                err=torch.zeros(1, dtype=torch.int32, device="cuda"))
+
+
+def _offset(torch, t, n):
+    """A copy of t that starts n elements behind a 16-byte boundary."""
+    flat = torch.zeros(t.numel() + 16, dtype=t.dtype, device="cuda")
+    v = flat[n:n + t.numel()].view(t.shape)
+    v.copy_(t)
+    return v
+
+
+@pytest.mark.parametrize("off", [1, 2, 3])
+def test_bias_as_a_slice_of_a_flat_parameter_buffer(off):
+    torch, lib, p, st = _sg()
+    members, B, K, N = 2, 128, 64, 128
+    d = _layer(torch, members, B, K, N)
+    b = _offset(torch, d["b"], off)
+    assert b.data_ptr() % 16 == 4 * off
+    out = []
+    for bias in (d["b"], b):
+        Y, m, s = torch.zeros(members, B, N, device="cuda"), torch.zeros(B, N, device="cuda"), torch.zeros(B, device="cuda")
+        assert lib.luna_sg_linear_fwd(p(d["X"]), B * K, p(d["W"]), p(bias), B, K, N, 1, None, None, p(Y), members, p(d["err"]), st) == 0
+        assert lib.luna_sg_linear_ensemble(p(d["X"]), B * K, p(d["W"]), p(bias), B, K, N, N, p(m), p(s), members, p(d["err"]), st) == 0
+        out.append((Y, m, s))
+    torch.cuda.synchronize()
+    assert int(d["err"].item()) == 0
+    assert all(torch.equal(x, y) for x, y in zip(*out))
+
+
+def test_misaligned_outputs_are_refused():
+    """Return codes only: nothing is launched."""
+    torch, lib, p, st = _sg()
+    members, B, K, N = 1, 128, 128, 128
+    d = _layer(torch, members, B, K, N)
+    bf = torch.bfloat16
+    big = torch.zeros(B * N + 64, device="cuda")
+    q = lambda nbytes: ctypes.c_void_p(big.data_ptr() + nbytes)
+    X, W, b, dZ, Zp, err = (p(d[k]) for k in ("X", "W", "b", "dZ", "Zp", "err"))
+    for k in (4, 8):
+        for Y, Z, Yf in ((q(k), None, None), (None, q(k), None), (None, None, q(k))):
+            assert lib.luna_sg_linear_fwd(X, B * K, W, b, B, K, N, 1, Y, Z, Yf, members, err, st) == 16
+        assert lib.luna_sg_linear_bwd_data(dZ, W, Zp, B, K, N, q(k), members, err, st) == 16
+        assert lib.luna_sg_linear_bwd_data(dZ, W, q(k), B, K, N, q(0), members, err, st) == 16
+        assert lib.luna_sg_linear_bwd_weight(dZ, X, B * K, B, K, N, q(k), b, members, err, st) == 16
+    assert lib.luna_sg_linear_fwd(X, B * K, W, q(2), B, K, N, 1, None, None, q(16), members, err, st) == 16
+    torch.cuda.synchronize()
+    assert not big.any()
