@@ -23,7 +23,10 @@ extern "C" {
  * BF16 (member stride sX, 0 to share one input), W [N x K] BF16 (stride N*K), b [N] FP32
  * (stride N); outputs [B x N] (stride B*N): Y BF16, Zout BF16, Yf FP32, each may be NULL.
  * Here and in the backward products outputs and Zprev are 16-byte aligned (else
- * LUNA_ERR_BAD_ARG, nothing is launched); b and db need the 4 bytes of an FP32 value. */
+ * LUNA_ERR_BAD_ARG, nothing is launched); b and db need the 4 bytes of an FP32 value. Inputs: X
+ * and W here and dZ of the data product 16 bytes with a stride of a multiple of 8, W of the data
+ * product and dZ and X of the weight product 4 bytes with an even stride (off 16 bytes or 8
+ * elements they are copied to stream-ordered memory first); strides may be negative. */
 int luna_sg_linear_fwd(const void* X, long long sX, const void* W, const float* b, int B, int K, int N, int act,
                        void* Y, void* Zout, float* Yf, int members, int* err, void* stream);
 /* Backward through the layer's input: dXpre = (dZ W) * silu'(Zprev), [B x K] BF16. */

@@ -72,3 +72,40 @@ def test_misaligned_outputs_are_refused():
     assert lib.luna_sg_linear_fwd(X, B * K, W, q(2), B, K, N, 1, None, None, q(16), members, err, st) == 16
     torch.cuda.synchronize()
     assert not big.any()
+
+
+@pytest.mark.parametrize("off,gap", [(0, 2), (2, 0), (4, 6), (6, 0)])
+def test_backward_operands_at_four_byte_alignment(off, gap):
+    """dZ, X and W of the transposed roles as slices of larger buffers (`off` elements behind a 16-byte
+    boundary) and X with a member stride of an even number of elements."""
+    torch, lib, p, st = _sg()
+    members, B, K, N = 2, 128, 128, 256
+    d = _layer(torch, members, B, K, N)
+    Xb = torch.zeros(members * (B * K + gap) + 16, dtype=torch.bfloat16, device="cuda")
+    for m in range(members):
+        Xb[off + m * (B * K + gap):][:B * K].copy_(d["X"][m].flatten())
+    moved = dict(X=(Xb[off:], B * K + gap), dZ=_offset(torch, d["dZ"], off), W=_offset(torch, d["W"], off))
+    out = []
+    for X, sX, dZ, W in ((d["X"], B * K, d["dZ"], d["W"]), (*moved["X"], moved["dZ"], moved["W"])):
+        dX, dW, db = (torch.zeros(members, B, K, device="cuda", dtype=torch.bfloat16), torch.zeros(members, N, K, device="cuda"),
+                      torch.zeros(members, N, device="cuda"))
+        assert lib.luna_sg_linear_bwd_data(p(d["dZ"]), p(W), p(d["Zp"]), B, K, N, p(dX), members, p(d["err"]), st) == 0
+        assert lib.luna_sg_linear_bwd_weight(p(dZ), p(X), sX, B, K, N, p(dW), p(db), members, p(d["err"]), st) == 0
+        out.append((dX, dW, db))
+    torch.cuda.synchronize()
+    assert int(d["err"].item()) == 0 and out[0][1].any()
+    assert all(torch.equal(x, y) for x, y in zip(*out))
+
+
+def test_members_in_reverse_order():
+    """A negative member stride: member z reads the matrix before member z - 1's."""
+    torch, lib, p, st = _sg()
+    members, B, K, N = 3, 128, 64, 128
+    d = _layer(torch, members, B, K, N)
+    Y = torch.zeros(2, members, B, N, device="cuda")
+    last = ctypes.c_void_p(d["X"][-1].data_ptr())
+    assert lib.luna_sg_linear_fwd(last, -B * K, p(d["W"]), p(d["b"]), B, K, N, 1, None, None, p(Y[0]), members, p(d["err"]), st) == 0
+    X = d["X"].flip(0).contiguous()
+    assert lib.luna_sg_linear_fwd(p(X), B * K, p(d["W"]), p(d["b"]), B, K, N, 1, None, None, p(Y[1]), members, p(d["err"]), st) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(Y[0], Y[1]) and int(d["err"].item()) == 0
