@@ -109,3 +109,23 @@ def test_members_in_reverse_order():
     assert lib.luna_sg_linear_fwd(p(X), B * K, p(d["W"]), p(d["b"]), B, K, N, 1, None, None, p(Y[1]), members, p(d["err"]), st) == 0
     torch.cuda.synchronize()
     assert torch.equal(Y[0], Y[1]) and int(d["err"].item()) == 0
+
+
+@pytest.mark.parametrize("B,nf", [(1, 1), (65, 252), (4095, 129), (4096, 128), (4100, 128), (22000, 24), (131072, 23), (5000, 896), (70, 897), (4097, 2000)])
+def test_features_of_every_width(B, nf):
+    """Both kernels at the edges of their rule, and rows that do not fit in shared memory. Bound: the
+    projection's eight rounded products and sums (|f . x| < 60: 16 2^-24 60 of a turn, times 2 pi 3.6e-4)
+    and the rounding to BF16 (2^-9)."""
+    torch, lib, p, st = _sg()
+    g = torch.Generator(device="cuda").manual_seed(nf)
+    x, f = torch.randn(B, 8, device="cuda", generator=g), torch.randn(nf, 8, device="cuda", generator=g)
+    ld = 8 + 2 * nf
+    out = torch.full((B, ld), 9.0, device="cuda", dtype=torch.bfloat16)
+    assert lib.luna_sg_features(p(x), B, p(f), nf, p(out), ld, st) == 0
+    torch.cuda.synchronize()
+    d = x.double() @ f.double().T
+    assert d.abs().max() < 60
+    a = 2 * torch.pi * (d - d.round())
+    assert torch.equal(out[:, :8], x.to(torch.bfloat16))
+    assert (out[:, 8:8 + nf].double() - a.sin()).abs().max() < 2.0 ** -9 + 4e-4
+    assert (out[:, 8 + nf:].double() - a.cos()).abs().max() < 2.0 ** -9 + 4e-4
