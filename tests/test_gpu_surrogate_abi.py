@@ -129,3 +129,20 @@ def test_features_of_every_width(B, nf):
     assert torch.equal(out[:, :8], x.to(torch.bfloat16))
     assert (out[:, 8:8 + nf].double() - a.sin()).abs().max() < 2.0 ** -9 + 4e-4
     assert (out[:, 8 + nf:].double() - a.cos()).abs().max() < 2.0 ** -9 + 4e-4
+
+
+@pytest.mark.parametrize("B,N,nspec,members", [(1, 512, 512, 12), (2048, 768, 100, 3), (2049, 768, 100, 3), (300, 511, 511, 2), (300, 513, 257, 5),
+                                               (77, 4099, 0, 1), (130, 7, 7, 40)])
+def test_statistics_with_a_warp_or_a_block_a_row(B, N, nspec, members):
+    """Mean and spread against 64-bit values: the sums of `members` FP32 terms and one division within
+    members 2^-23 of the sum of magnitudes, a variance within 4 members 2^-23 of the mean square."""
+    torch, lib, p, st = _sg()
+    Y = torch.randn(members, B, N, device="cuda", generator=torch.Generator(device="cuda").manual_seed(N)) + 1
+    mean, spread = torch.full((B, N), 7.0, device="cuda"), torch.full((B,), 7.0, device="cuda")
+    assert lib.luna_sg_ensemble(p(Y), members, B, N, nspec, p(mean), p(spread), st) == 0
+    torch.cuda.synchronize()
+    d = Y.double()
+    assert ((mean - d.mean(0)).abs() <= members * 2.0 ** -23 * d.abs().mean(0)).all()
+    var = d.var(0, unbiased=False)[:, :nspec].amax(1) if nspec and members > 1 else torch.zeros(B, device="cuda").double()
+    msq = (d ** 2).mean(0)[:, :max(nspec, 1)].amax(1)
+    assert ((spread.double() ** 2 - var).abs() <= 4 * members * 2.0 ** -23 * msq).all()
