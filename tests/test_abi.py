@@ -196,3 +196,14 @@ def test_julia_binding_solveopts_call_passes_every_field():
     assert calls
     for c in calls:
         assert len([a for a in c.split(",") if a.strip()]) == len(_lib.SolveOpts._fields_), c
+
+
+def test_loss_of_no_members_is_refused():
+    """luna_sg_mse sizes its grid by the number of members: none is an error code, not a division by
+    zero on the host (run in a process of its own, which would end by a signal)."""
+    import sys
+    from luna_b200 import surrogate
+    code = ("import ctypes, sys; lib = ctypes.CDLL(sys.argv[1]); f = lib.luna_sg_mse; v, i, l = ctypes.c_void_p, ctypes.c_int, "
+            "ctypes.c_longlong; f.argtypes = [v, v, l, i, i, v, v, i, v]; print([f(None, None, 0, 128, 128, None, None, m, None) for m in (0, -1)])")
+    r = subprocess.run([sys.executable, "-c", code, surrogate.LIB_PATH], capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.strip() == "[18, 18]", (r.returncode, r.stdout, r.stderr)
