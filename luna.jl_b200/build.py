@@ -27,7 +27,8 @@ PEAKS_OUT = os.path.join(HERE, "libluna_peaks.so")
 # the learned surrogate's training and inference kernels (include/luna_surrogate.h)
 SG_SRC = os.path.join(HERE, "csrc", "surrogate.cu")
 SG_DEPS = [SG_SRC, os.path.join(HERE, "csrc", "tc_gemm.cuh"), os.path.join(HERE, "csrc", "common.cuh"),
-           os.path.join(HERE, "..", "include", "luna_surrogate.h")]
+           os.path.join(HERE, "..", "include", "luna_surrogate.h"),
+           os.path.join(HERE, "..", "include", "luna_surrogate_ensemble.h")]
 SG_OUT = os.path.join(HERE, "libluna_surrogate.so")
 
 

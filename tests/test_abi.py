@@ -207,3 +207,12 @@ def test_loss_of_no_members_is_refused():
             "ctypes.c_longlong; f.argtypes = [v, v, l, i, i, v, v, i, v]; print([f(None, None, 0, 128, 128, None, None, m, None) for m in (0, -1)])")
     r = subprocess.run([sys.executable, "-c", code, surrogate.LIB_PATH], capture_output=True, text=True)
     assert r.returncode == 0 and r.stdout.strip() == "[18, 18]", (r.returncode, r.stdout, r.stderr)
+
+
+def test_every_surrogate_symbol_is_declared():
+    """The C symbols that libluna_surrogate.so exports are those of its two headers."""
+    from luna_b200 import surrogate
+    hdr = "".join((ROOT / "include" / h).read_text() for h in ("luna_surrogate.h", "luna_surrogate_ensemble.h"))
+    names = set(re.findall(r"\b(luna_sg_\w+)\s*\(", hdr))
+    out = subprocess.run(["nm", "-D", "--defined-only", surrogate.LIB_PATH], capture_output=True, text=True, check=True).stdout
+    assert {l.split()[-1] for l in out.splitlines() if "luna_sg_" in l and l.split()[-1].startswith("luna_sg_")} == names
