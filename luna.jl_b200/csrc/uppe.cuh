@@ -349,7 +349,7 @@ __device__ __forceinline__ void rates_f64(const LunaResp& r, const double* E, in
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
         aE[s] = fabs(E[s]);
-        in[s] = !(aE[s] < lo) && aE[s] != 0.0;
+        in[s] = !(aE[s] < lo) && (ppt || aE[s] != 0.0);  // (a table may begin at a zero field)
         out[s] = 0.0;
         any = any || in[s];
     }
