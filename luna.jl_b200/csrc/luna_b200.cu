@@ -548,6 +548,14 @@ int max_smem_optin() {
     return v - 3072;  // leave room for the kernels' static shared memory
 }
 
+// Raises a kernel's limit of dynamic shared memory to the device's. Never to less: the limit is the
+// kernel's, whoever launches it, and a caller of small grids must not lower it between another's
+// creation or check and its launch.
+template <typename K>
+cudaError_t allow_smem(K kern) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin());
+}
+
 template <typename Rl>
 size_t smem_wanted(const LunaInst& I) {
     const size_t c = sizeof(cpx<Rl>);
@@ -723,8 +731,7 @@ void free_all(std::vector<void*>& allocs) {
 }
 
 // Clusters of R CTAs of `kern` (sm bytes of dynamic shared memory) that fit on the device at once;
-// raises the kernel's limits (to the device's, so that callers of different sizes never lower each
-// other's).
+// raises the kernel's limits.
 template <typename K>
 int max_clusters(K kern, int R, int sm) {
     int ncl = 0;
@@ -739,7 +746,7 @@ int max_clusters(K kern, int R, int sm) {
     cfg.dynamicSmemBytes = sm;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin()) != cudaSuccess ||
+    if (allow_smem(kern) != cudaSuccess ||
         (R > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
         cudaOccupancyMaxActiveClusters(&ncl, kern, &cfg) != cudaSuccess) {
         cudaGetLastError();
@@ -831,8 +838,6 @@ int dist_setup(luna_batch* b, const luna_solve_opts* opts, int nsm) {
     }
     if (dl.empty()) return LUNA_OK;
     const int sm = (int)std::max<size_t>((size_t)b->smem, dsm_b);
-    if (cudaFuncSetAttribute(solve_kernel<Rl, Rl>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) != cudaSuccess)
-        return fail(LUNA_ERR_CUDA, "batch_create: cannot set shared memory size (distributed solver)");
     const int ncl = max_clusters(solve_kernel_dist<Rl, Rl, DIST_R>, DIST_R, sm);
     if (ncl < 1) return LUNA_OK;
     const int ncl16 = dl16.empty() ? 0 : max_clusters(solve_kernel_dist<Rl, Rl, DIST_R_BIG>, DIST_R_BIG, sm);
@@ -1183,11 +1188,11 @@ static int launch_rhs(luna_plan* p, const double2* Ew, double2* nl, cudaStream_t
                                                                              : launch_rhs_dist<4>(p, Ew, nl, st, tw);
         }
         int sm = (int)std::min<size_t>(smem_wanted<double>(p->proto), (size_t)maxs);
-        CK(cudaFuncSetAttribute(rhs_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+        CK(allow_smem(rhs_kernel<double>));
         rhs_kernel<double><<<1, LUNA_BLOCK, sm, st>>>(p->d_inst, Ew, nl, tw.d, sm, p->d_status, z);
     } else {
         int sm = (int)std::min<size_t>(smem_wanted<float>(p->proto), (size_t)maxs);
-        CK(cudaFuncSetAttribute(rhs_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+        CK(allow_smem(rhs_kernel<float>));
         rhs_kernel<float><<<1, LUNA_BLOCK, sm, st>>>(p->d_inst, Ew, nl, tw.f, sm, p->d_status, z);
     }
     CK(cudaGetLastError());
@@ -1430,11 +1435,11 @@ int luna_b200_batch_create(luna_plan* const* plans, int n, const luna_solve_opts
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     if (prec == LUNA_PREC_FP64) {
-        if (cudaFuncSetAttribute(solve_kernel<double, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, b->smem) != cudaSuccess)
+        if (allow_smem(solve_kernel<double, double>) != cudaSuccess)
             return bail(fail(LUNA_ERR_CUDA, "batch_create: cannot set shared memory size"));
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, solve_kernel<double, double>, LUNA_BLOCK, b->smem);
     } else {
-        if (cudaFuncSetAttribute(solve_kernel<float, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, b->smem) != cudaSuccess)
+        if (allow_smem(solve_kernel<float, float>) != cudaSuccess)
             return bail(fail(LUNA_ERR_CUDA, "batch_create: cannot set shared memory size"));
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, solve_kernel<float, float>, LUNA_BLOCK, b->smem);
     }
@@ -1462,7 +1467,7 @@ int luna_b200_batch_create(luna_plan* const* plans, int n, const luna_solve_opts
         }
         std::stable_sort(reg.begin(), reg.end(), [&](int a, int c) { return cost[a] > cost[c]; });
         if (!big.empty()) {
-            if (cudaFuncSetAttribute(solve_kernel_cl<float, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, b->smem) != cudaSuccess)
+            if (allow_smem(solve_kernel_cl<float, float>) != cudaSuccess)
                 return bail(fail(LUNA_ERR_CUDA, "batch_create: cannot set shared memory size (clusters)"));
             cudaLaunchConfig_t cfg = {};
             cudaLaunchAttribute at[1];
@@ -1807,10 +1812,9 @@ int rad_column_setup(luna_radial_plan* p) {
         p->gstride = align_up(gscr_bytes<Rl>(I), 256);
         if (dalloc(p->allocs, &p->gscr, p->gstride * p->Nr)) return LUNA_ERR_CUDA;
     }
-    // the device maximum, so that plans of different sizes never lower each other's limit
-    CK(cudaFuncSetAttribute(rad_column_kernel<Rl>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs));
-    CK(cudaFuncSetAttribute(rad_post_kernel<Rl, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs));
-    CK(cudaFuncSetAttribute(rad_post_kernel<Rl, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs));
+    CK(allow_smem(rad_column_kernel<Rl>));
+    CK(allow_smem(rad_post_kernel<Rl, double>));
+    CK(allow_smem(rad_post_kernel<Rl, float>));
     return LUNA_OK;
 }
 
@@ -2427,11 +2431,11 @@ int modal_setup(luna_modal_plan* p) {
             if (!modal_dist_setup<16>(p) && !modal_dist_setup<8>(p)) modal_dist_setup<4>(p);
         }
     }
-    CK(cudaFuncSetAttribute(modal_time_kernel<Rl>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs));
-    CK(cudaFuncSetAttribute(modal_node_kernel<Rl>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs));
-    CK(cudaFuncSetAttribute(modal_level_kernel<Rl>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs));
-    CK(cudaFuncSetAttribute(rad_post_kernel<Rl, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs));
-    CK(cudaFuncSetAttribute(rad_post_kernel<Rl, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs));
+    CK(allow_smem(modal_time_kernel<Rl>));
+    CK(allow_smem(modal_node_kernel<Rl>));
+    CK(allow_smem(modal_level_kernel<Rl>));
+    CK(allow_smem(rad_post_kernel<Rl, double>));
+    CK(allow_smem(rad_post_kernel<Rl, float>));
     return LUNA_OK;
 }
 
@@ -2682,11 +2686,11 @@ extern "C" int luna_b200_rhs_device_noalloc(luna_plan* p, double* nl_dev, const 
     cudaStream_t st = (cudaStream_t)stream;
     if (p->precision == LUNA_PREC_FP64) {
         int sm = (int)std::min<size_t>(smem_wanted<double>(I), (size_t)maxs);
-        CK(cudaFuncSetAttribute(rhs_kernel_noalloc<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+        CK(allow_smem(rhs_kernel_noalloc<double>));
         rhs_kernel_noalloc<double><<<1, LUNA_BLOCK, sm, st>>>(I, (const double2*)Ew_dev, (double2*)nl_dev, tw.d, sm, status_dev);
     } else {
         int sm = (int)std::min<size_t>(smem_wanted<float>(I), (size_t)maxs);
-        CK(cudaFuncSetAttribute(rhs_kernel_noalloc<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+        CK(allow_smem(rhs_kernel_noalloc<float>));
         rhs_kernel_noalloc<float><<<1, LUNA_BLOCK, sm, st>>>(I, (const double2*)Ew_dev, (double2*)nl_dev, tw.f, sm, status_dev);
     }
     CK(cudaGetLastError());
