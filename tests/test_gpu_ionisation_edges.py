@@ -1,6 +1,7 @@
 """Ionisation rates at the edges of their range, in the kernels of one CTA (the allocation-free entry
 point) and of clusters of 4, 8 and 16 (rhs_device), against the FP64 oracle.
 """
+import copy
 import ctypes
 
 import luna_b200_loader  # registers the luna.jl_b200 package
@@ -50,7 +51,8 @@ def test_table_that_begins_at_a_zero_field(trange, monkeypatch):
     """A constant rate from E = 0 on, on a field whose every fourth sample is an exact zero (1 +
     cos(pi n / 2) on the oversampled grid): those samples ionise like the others."""
     p = _problem(trange)
-    r = next(q for q in p.transform.resp if q.kind == "plasma").ratefunc
+    plasma = next(q for q in p.transform.resp if q.kind == "plasma")
+    r = plasma.ratefunc = copy.copy(plasma.ratefunc)  # (tables are shared between problems)
     n, top = len(r.x), r.x[-1]
     r.x, r.y, r.D = np.linspace(0.0, top, n), np.full(n, np.log(1e13)), np.zeros(n)
     r.Emin = 0.0
