@@ -569,10 +569,18 @@ size_t smem_wanted(const LunaInst& I) {
 
 }  // namespace
 
+// Device memory of one object; kept: from the pool and back to it, all work on it on streams of the
+// owner's and every copy into it on `stream`.
+struct DevMem {
+    std::vector<void*> list;
+    bool kept = false;
+    cudaStream_t stream = nullptr;
+};
+
 struct luna_plan {
     int precision = 0;
     LunaInst proto{};
-    std::vector<void*> allocs;
+    DevMem allocs;
     bool has_raman = false;
     void* d_hbuf = nullptr;      // FP64 work buffer of the Raman spectrum build ([No] complex)
     LunaGrad* d_grad = nullptr;  // pressure gradient (device copy), or null
@@ -603,7 +611,7 @@ struct luna_batch {
     int* d_reg = nullptr;
     int* d_cl_counters = nullptr;  // [0] big, [1] regular, [2] error flag
     std::vector<int> big, reg;     // host copies of the two lists
-    std::vector<void*> allocs;
+    DevMem allocs;
     std::vector<double2*> y0buf;  // per instance y (holds y0 before the run)
     std::vector<double2*> ybuf, ynbuf;
     std::vector<double*> steplogs;
@@ -631,12 +639,13 @@ struct luna_batch {
 
 namespace {
 
-// Device memory of plans, batches and solves. Blocks that an object gives back are kept for the next
-// one: a solve on a plan that stays takes 20 to 30 buffers, and allocating and freeing them was
-// 1.7 ms of an 11 ms propagation and 3.5 ms of a 10 ms radial one. Kept are at most
-// POOL_KEEP bytes in blocks of at most POOL_BLOCK, and nothing once the last object is gone
-// (or when an allocation fails). A block is given back after the device has finished all
-// work, cleared like a fresh one, so the next owner may use it on any stream and thread.
+// Device memory of batches and solves. Blocks that one gives back are kept for the next: a solve on a
+// plan that stays takes 20 to 30 buffers, and allocating and freeing them was 1.7 ms of an 11 ms
+// propagation and 3.5 ms of a 10 ms radial one. Kept are at most POOL_KEEP bytes in blocks of at most
+// POOL_BLOCK, and nothing once the last plan and batch are gone (or when an allocation fails). The
+// owner's work is on streams of its own, so giving back waits for these alone: not for the device,
+// which would hold up a caller behind other threads' work and is an error while any stream is captured.
+// The lock covers the books, not what waits. Blocks are cleared like fresh ones.
 struct DevPool {
     static constexpr size_t POOL_KEEP = (size_t)64 << 20, POOL_BLOCK = (size_t)16 << 20;
     struct Block {
@@ -646,16 +655,33 @@ struct DevPool {
     std::mutex m;
     std::map<void*, Block> live;
     std::multimap<size_t, std::pair<int, void*>> idle;  // by size
-    size_t held = 0;
+    size_t held = 0;                                     // bytes idle or being cleared
+    int objects = 0;                                     // plans and batches
 
     static DevPool& get() {
         static DevPool* p = new DevPool;  // never destroyed: objects may be freed at exit
         return *p;
     }
-    void trim() {  // with the lock held
-        for (auto& b : idle) cudaFree(b.second.second);
+    std::vector<void*> idle_blocks() {  // taken off the books, with the lock held
+        std::vector<void*> out;
+        for (auto& b : idle) {
+            out.push_back(b.second.second);
+            held -= b.first;
+        }
         idle.clear();
-        held = 0;
+        return out;
+    }
+    void hold() {
+        std::lock_guard<std::mutex> lk(m);
+        ++objects;
+    }
+    void drop() {
+        std::vector<void*> out;
+        {
+            std::lock_guard<std::mutex> lk(m);
+            if (--objects == 0) out = idle_blocks();
+        }
+        for (void* p : out) cudaFree(p);
     }
     cudaError_t take(void** out, size_t bytes) {
         const size_t unit = bytes <= ((size_t)1 << 20) ? 512 : (size_t)1 << 16;
@@ -663,71 +689,105 @@ struct DevPool {
         int dev = 0;
         cudaError_t e = cudaGetDevice(&dev);
         if (e != cudaSuccess) return e;
-        std::lock_guard<std::mutex> lk(m);
-        for (auto it = idle.lower_bound(n); it != idle.end() && it->first <= n + n / 4; ++it) {
-            if (it->second.first != dev) continue;
-            *out = it->second.second;
-            held -= it->first;
-            live[*out] = Block{it->first, dev};
-            idle.erase(it);
-            return cudaSuccess;
-        }
-        e = cudaMalloc(out, n);
-        if (e == cudaErrorMemoryAllocation && !idle.empty()) {
-            cudaGetLastError();
-            trim();
-            e = cudaMalloc(out, n);
-        }
-        if (e == cudaSuccess) live[*out] = Block{n, dev};
-        return e;
-    }
-    void give(std::vector<void*>& list) {
-        if (list.empty()) return;
-        std::lock_guard<std::mutex> lk(m);
-        int dev = 0;
-        // (a device in an error state keeps nothing)
-        bool keep = cudaGetDevice(&dev) == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess;
-        std::vector<std::pair<size_t, void*>> kept;
-        for (void* p : list) {
-            auto it = live.find(p);
-            if (it == live.end()) continue;
-            const Block b = it->second;
-            live.erase(it);
-            if (keep && b.dev == dev && b.size <= POOL_BLOCK && held + b.size <= POOL_KEEP && cudaMemset(p, 0, b.size) == cudaSuccess) {
-                kept.push_back({b.size, p});
-                held += b.size;
-            } else {
-                cudaFree(p);
+        {
+            std::lock_guard<std::mutex> lk(m);
+            for (auto it = idle.lower_bound(n); it != idle.end() && it->first <= n + n / 4; ++it) {
+                if (it->second.first != dev) continue;
+                *out = it->second.second;
+                held -= it->first;
+                live[*out] = Block{it->first, dev};
+                idle.erase(it);
+                return cudaSuccess;
             }
         }
-        keep = kept.empty() || cudaDeviceSynchronize() == cudaSuccess;
-        for (auto& k : kept) idle.insert({k.first, {dev, k.second}});
-        if (live.empty() || !keep) trim();
+        e = cudaMalloc(out, n);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            std::vector<void*> back;
+            {
+                std::lock_guard<std::mutex> lk(m);
+                back = idle_blocks();
+            }
+            for (void* p : back) cudaFree(p);
+            e = cudaMalloc(out, n);
+        }
+        if (e == cudaSuccess) {
+            std::lock_guard<std::mutex> lk(m);
+            live[*out] = Block{n, dev};
+        }
+        return e;
+    }
+    // s: the owner's stream, the only one with work on the blocks
+    void give(std::vector<void*>& list, cudaStream_t s) {
+        if (list.empty()) return;
+        int dev = 0;
+        // (a device in an error state keeps nothing)
+        bool keep = s && cudaStreamSynchronize(s) == cudaSuccess && cudaGetDevice(&dev) == cudaSuccess;
+        std::vector<std::pair<size_t, void*>> kept;
+        std::vector<void*> out;
+        {
+            std::lock_guard<std::mutex> lk(m);
+            for (void* p : list) {
+                auto it = live.find(p);
+                const Block b = it->second;
+                live.erase(it);
+                if (keep && b.dev == dev && b.size <= POOL_BLOCK && held + b.size <= POOL_KEEP) {
+                    kept.push_back({b.size, p});
+                    held += b.size;
+                } else {
+                    out.push_back(p);
+                }
+            }
+        }
+        for (auto& k : kept) keep = keep && cudaMemsetAsync(k.second, 0, k.first, s) == cudaSuccess;
+        keep = (kept.empty() || cudaStreamSynchronize(s) == cudaSuccess) && keep;
+        {
+            std::lock_guard<std::mutex> lk(m);
+            for (auto& k : kept) {
+                if (keep) {
+                    idle.insert({k.first, {dev, k.second}});
+                } else {
+                    held -= k.first;
+                    out.push_back(k.second);
+                }
+            }
+        }
+        for (void* p : out) cudaFree(p);
     }
 };
 
 template <typename T>
-int dalloc(std::vector<void*>& allocs, T** p, size_t bytes) {
+int dalloc(DevMem& m, T** p, size_t bytes) {
     void* q = nullptr;
-    CK(DevPool::get().take(&q, bytes > 0 ? bytes : 16));
-    allocs.push_back(q);
+    if (bytes < 1) bytes = 16;
+    CK(m.kept ? DevPool::get().take(&q, bytes) : cudaMalloc(&q, bytes));
+    m.list.push_back(q);
     *p = reinterpret_cast<T*>(q);
     return LUNA_OK;
 }
 
+// host array into the object's memory: complete on return, or (kept memory) in the order of its stream
 template <typename T>
-int upload(std::vector<void*>& allocs, const T* src, size_t n, const T** dst) {
-    T* p = nullptr;
-    int rc = dalloc(allocs, &p, n * sizeof(T));
-    if (rc) return rc;
-    CK(cudaMemcpy(p, src, n * sizeof(T), cudaMemcpyHostToDevice));
-    *dst = p;
+int h2d(DevMem& m, T* dst, const void* src, size_t bytes) {
+    if (m.kept) CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, m.stream));
+    else CK(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
     return LUNA_OK;
 }
 
-void free_all(std::vector<void*>& allocs) {
-    DevPool::get().give(allocs);
-    allocs.clear();
+template <typename T>
+int upload(DevMem& m, const T* src, size_t n, const T** dst) {
+    T* p = nullptr;
+    int rc = dalloc(m, &p, n * sizeof(T));
+    if (!rc) rc = h2d(m, p, src, n * sizeof(T));
+    *dst = p;
+    return rc;
+}
+
+void free_all(DevMem& m) {
+    if (m.kept) DevPool::get().give(m.list, m.stream);
+    else
+        for (void* p : m.list) cudaFree(p);
+    m.list.clear();
 }
 
 // Clusters of R CTAs of `kern` (sm bytes of dynamic shared memory) that fit on the device at once;
@@ -810,9 +870,10 @@ int dist_partition(luna_batch* b, const double* pr) {
     b->dist16_grid = DIST_R_BIG * n16;
     b->dist_grid = DIST_R * std::min(b->ncl_max, b->ndist);
     b->reg_grid = std::max(0, std::min(b->nreg, b->nsm - DIST_R * room - b->dist16_grid));
-    if (b->ndist > 0) CK(cudaMemcpy(b->d_dist, b->dist.data(), sizeof(int) * b->ndist, cudaMemcpyHostToDevice));
-    if (b->ndist16 > 0) CK(cudaMemcpy(b->d_dist16, b->dist16.data(), sizeof(int) * b->ndist16, cudaMemcpyHostToDevice));
-    if (b->nreg > 0) CK(cudaMemcpy(b->d_reg, b->reg.data(), sizeof(int) * b->nreg, cudaMemcpyHostToDevice));
+    if ((b->ndist > 0 && h2d(b->allocs, b->d_dist, b->dist.data(), sizeof(int) * b->ndist)) ||
+        (b->ndist16 > 0 && h2d(b->allocs, b->d_dist16, b->dist16.data(), sizeof(int) * b->ndist16)) ||
+        (b->nreg > 0 && h2d(b->allocs, b->d_reg, b->reg.data(), sizeof(int) * b->nreg)))
+        return LUNA_ERR_CUDA;
     return LUNA_OK;
 }
 
@@ -1114,6 +1175,7 @@ int luna_b200_plan_create(const luna_grid_desc* g, const luna_resp_desc* resps, 
         }
     }
 #undef UP
+    DevPool::get().hold();
     *out = p;
     return LUNA_OK;
 }
@@ -1123,6 +1185,7 @@ void luna_b200_plan_destroy(luna_plan* p) {
     if (p->stream) cudaStreamDestroy(p->stream);
     free_all(p->allocs);
     delete p;
+    DevPool::get().drop();
 }
 
 // CTAs of one FP64 right-hand side: the largest cluster that leaves each CTA 512 samples or sample
@@ -1353,11 +1416,24 @@ int luna_b200_batch_create(luna_plan* const* plans, int n, const luna_solve_opts
     b->steplogs.assign(n, nullptr);
     b->zsave_own.assign(n, nullptr);
     const size_t kel = (prec == LUNA_PREC_FP64) ? sizeof(double2) : sizeof(float2);
+    DevPool::get().hold();
     auto bail = [&](int rc) {
-        free_all(b->allocs);
-        delete b;
+        luna_b200_batch_destroy(b);
         return rc;
     };
+    // where SMs come free, the widest clusters are placed first, single CTAs last
+    int plo = 0, phi = 0;
+    cudaDeviceGetStreamPriorityRange(&plo, &phi);
+    if (cudaStreamCreateWithPriority(&b->stream, cudaStreamNonBlocking, std::min(plo, phi + 1)) != cudaSuccess ||
+        cudaStreamCreateWithPriority(&b->stream2, cudaStreamNonBlocking, plo) != cudaSuccess ||
+        cudaStreamCreateWithPriority(&b->stream3, cudaStreamNonBlocking, phi) != cudaSuccess ||
+        cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess ||
+        cudaEventCreateWithFlags(&b->evf, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&b->evj, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&b->evj3, cudaEventDisableTiming) != cudaSuccess)
+        return bail(fail(LUNA_ERR_CUDA, "batch_create: stream/event creation failed"));
+    b->allocs.kept = true;
+    b->allocs.stream = b->stream;
     if (opts->saveN > 0) {
         const double* zs = nullptr;
         if (upload(b->allocs, opts->zsave, (size_t)opts->saveN, &zs)) return bail(LUNA_ERR_CUDA);
@@ -1504,17 +1580,6 @@ int luna_b200_batch_create(luna_plan* const* plans, int n, const luna_solve_opts
             }
         }
     }
-    // where SMs come free, the widest clusters are placed first, single CTAs last
-    int plo = 0, phi = 0;
-    cudaDeviceGetStreamPriorityRange(&plo, &phi);
-    if (cudaStreamCreateWithPriority(&b->stream, cudaStreamNonBlocking, std::min(plo, phi + 1)) != cudaSuccess ||
-        cudaStreamCreateWithPriority(&b->stream2, cudaStreamNonBlocking, plo) != cudaSuccess ||
-        cudaStreamCreateWithPriority(&b->stream3, cudaStreamNonBlocking, phi) != cudaSuccess ||
-        cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess ||
-        cudaEventCreateWithFlags(&b->evf, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&b->evj, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&b->evj3, cudaEventDisableTiming) != cudaSuccess)
-        return bail(fail(LUNA_ERR_CUDA, "batch_create: stream/event creation failed"));
     *out = b;
     return LUNA_OK;
 }
@@ -1667,8 +1732,9 @@ int luna_b200_batch_set_priority(luna_batch* b, const double* priority) {
     if (b->cl_grid == 0) return LUNA_OK;  // single list in index order
     std::stable_sort(b->big.begin(), b->big.end(), by);
     std::stable_sort(b->reg.begin(), b->reg.end(), by);
-    CK(cudaMemcpy(b->d_big, b->big.data(), sizeof(int) * b->big.size(), cudaMemcpyHostToDevice));
-    if (!b->reg.empty()) CK(cudaMemcpy(b->d_reg, b->reg.data(), sizeof(int) * b->reg.size(), cudaMemcpyHostToDevice));
+    if (h2d(b->allocs, b->d_big, b->big.data(), sizeof(int) * b->big.size()) ||
+        (!b->reg.empty() && h2d(b->allocs, b->d_reg, b->reg.data(), sizeof(int) * b->reg.size())))
+        return LUNA_ERR_CUDA;
     return LUNA_OK;
 }
 
@@ -1729,6 +1795,10 @@ int luna_b200_batch_set_replay(luna_batch* b, int i, const double* replay, long 
 
 void luna_b200_batch_destroy(luna_batch* b) {
     if (!b) return;
+    // a run that ended in an error may have left work behind
+    if (b->stream3) cudaStreamSynchronize(b->stream3);
+    if (b->stream2) cudaStreamSynchronize(b->stream2);
+    free_all(b->allocs);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
     if (b->evf) cudaEventDestroy(b->evf);
@@ -1737,8 +1807,8 @@ void luna_b200_batch_destroy(luna_batch* b) {
     if (b->stream3) cudaStreamDestroy(b->stream3);
     if (b->stream) cudaStreamDestroy(b->stream);
     if (b->stream2) cudaStreamDestroy(b->stream2);
-    free_all(b->allocs);
     delete b;
+    DevPool::get().drop();
 }
 
 int luna_b200_solve(luna_plan* p, const double* linop, double* y_inout, double z0, double dz0, double zmax,
@@ -1777,7 +1847,7 @@ struct luna_radial_plan {
     int Nw = 0, Nr = 0;
     luna_plan* col = nullptr;   // grid and responses of one radial column
     LunaInst* d_col = nullptr;  // device copy of the column descriptor
-    std::vector<void*> allocs;
+    DevMem allocs;
     const double* Mi = nullptr;      // [Nr*Nr] row-major QDHT k -> r
     const double* Mf = nullptr;      // [Nr*Nr] row-major QDHT r -> k
     // mixed precision: BF16 hi/lo splits of the QDHT matrices, pre-tiled for the
@@ -2113,7 +2183,7 @@ inline RadGrad plan_grad(const luna_modal_plan*) { return RadGrad{nullptr, nullp
 
 // Device buffers of one column solve (radial or modal transform).
 struct RadSolve {
-    std::vector<void*> allocs;
+    DevMem allocs;
     double2 *L = nullptr, *y = nullptr, *yn = nullptr, *e1 = nullptr, *saves = nullptr, *ofz = nullptr;
     void* k[7] = {};
     void** d_k = nullptr;
@@ -2137,7 +2207,11 @@ int col_solve(PlanT* p, XF&& xform, const char* who, const double* linop, double
     const size_t cb = sizeof(double2);
     const RadGrad G = plan_grad(p);
     if (!linop && !G.g) return fail(LUNA_ERR_BAD_ARG, std::string(who) + ": null linop");
+    if (!p->stream) CK(cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking));
+    const cudaStream_t s = p->stream;
     RadSolve S;
+    S.allocs.kept = true;
+    S.allocs.stream = s;
     if (G.g && dalloc(S.allocs, &S.ofz, cb * n)) return LUNA_ERR_CUDA;
     if (dalloc(S.allocs, &S.L, cb * n) || dalloc(S.allocs, &S.y, cb * n) || dalloc(S.allocs, &S.yn, cb * n) ||
         dalloc(S.allocs, &S.e1, cb * n) || dalloc(S.allocs, &S.st, sizeof(RadState)) ||
@@ -2148,14 +2222,15 @@ int col_solve(PlanT* p, XF&& xform, const char* who, const double* linop, double
     const int nblk = rad_grid(n);
     if (dalloc(S.allocs, &S.partial, sizeof(double) * 3 * nblk)) return LUNA_ERR_CUDA;
     if (o->saveN > 0) {
-        if (dalloc(S.allocs, &S.saves, cb * n * o->saveN) || dalloc(S.allocs, &S.zsave, sizeof(double) * o->saveN))
+        if (dalloc(S.allocs, &S.saves, cb * n * o->saveN) || dalloc(S.allocs, &S.zsave, sizeof(double) * o->saveN) ||
+            h2d(S.allocs, S.zsave, o->zsave, sizeof(double) * o->saveN))
             return LUNA_ERR_CUDA;
-        CK(cudaMemcpy(S.zsave, o->zsave, sizeof(double) * o->saveN, cudaMemcpyHostToDevice));
     }
     if (o->steplog_cap > 0 && dalloc(S.allocs, &S.steplog, sizeof(double) * 4 * o->steplog_cap)) return LUNA_ERR_CUDA;
     if (o->replay && o->nreplay > 0) {
-        if (dalloc(S.allocs, &S.replay, sizeof(double) * 2 * o->nreplay)) return LUNA_ERR_CUDA;
-        CK(cudaMemcpy(S.replay, o->replay, sizeof(double) * 2 * o->nreplay, cudaMemcpyHostToDevice));
+        if (dalloc(S.allocs, &S.replay, sizeof(double) * 2 * o->nreplay) ||
+            h2d(S.allocs, S.replay, o->replay, sizeof(double) * 2 * o->nreplay))
+            return LUNA_ERR_CUDA;
     }
     if (!p->h_fin) CK(cudaMallocHost(&p->h_fin, sizeof(int)));
     LunaInst I{};
@@ -2177,14 +2252,11 @@ int col_solve(PlanT* p, XF&& xform, const char* who, const double* linop, double
     I.steplog_cap = S.steplog ? o->steplog_cap : 0;
     I.replay = S.replay;
     I.nreplay = S.replay ? o->nreplay : 0;
-    CK(cudaMemcpy(S.opt, &I, sizeof(LunaInst), cudaMemcpyHostToDevice));
     // with a gas fill gradient L(z) is evaluated on the device and linop is ignored
-    if (!G.g) CK(cudaMemcpy(S.L, linop, cb * n, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(S.y, y_inout, cb * n, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(S.yn, y_inout, cb * n, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(S.d_k, S.k, sizeof(void*) * 7, cudaMemcpyHostToDevice));
-    if (!p->stream) CK(cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking));
-    cudaStream_t s = p->stream;
+    if (h2d(S.allocs, S.opt, &I, sizeof(LunaInst)) || (!G.g && h2d(S.allocs, S.L, linop, cb * n)) ||
+        h2d(S.allocs, S.y, y_inout, cb * n) || h2d(S.allocs, S.yn, y_inout, cb * n) ||
+        h2d(S.allocs, S.d_k, S.k, sizeof(void*) * 7))
+        return LUNA_ERR_CUDA;
     RadArgs a{p->Nw, p->Nr, S.L, G.g ? S.ofz : p->outfac, S.e1, S.st};
     const int eg = rad_grid(n);
     // FP64 without a gradient: a stage's store and the next stage's input in one launch
@@ -2279,7 +2351,7 @@ struct luna_modal_plan {
     double wlow = 0, rtol = 0, atol = 0, kerr = 0;
     luna_plan* col = nullptr;     // grid and responses of one point
     LunaInst* d_col = nullptr;
-    std::vector<void*> allocs;
+    DevMem allocs;
     const double2* outfac = nullptr;  // [Nr*Nw] crop * ωwin * norm!
     const double* ems = nullptr;      // [nslots*Nr*npol]
     const double* wts = nullptr;      // [nlevels*nslots]
