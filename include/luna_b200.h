@@ -396,6 +396,11 @@ void luna_b200_modal_plan_destroy(luna_modal_plan* plan);
 int luna_b200_modal_rhs(luna_modal_plan* plan, double* nl, const double* Ew, double z, int* nevals);
 int luna_b200_modal_rhs_device(luna_modal_plan* plan, double* nl_dev, const double* Ew_dev, double z,
                                void* stream);
+/* Full precision: the clusters of a transform wait for one another, at most `rounds` rounds of
+ * polling (default 2^24, some seconds; 0: not at all). When a wait runs out luna_b200_modal_rhs and
+ * luna_b200_modal_solve return LUNA_WAIT_TIMEOUT, and luna_b200_modal_rhs_device, which has no
+ * answer but its result, leaves NaN in the modes concerned. The plan stays usable. */
+int luna_b200_modal_set_wait(luna_modal_plan* plan, unsigned rounds);
 /* RK45.solve_precon driven by Luna.run (Luna.jl:358-391) for a modal problem: linop and
  * y_inout are Nw*nmodes complex (LinearOps.make_const_linop(grid, modes, λ0),
  * LinearOps.jl:401-415), saves [saveN*2*Nw*nmodes] doubles, steplog as for luna_b200_solve. */

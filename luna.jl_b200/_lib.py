@@ -110,7 +110,7 @@ EXPORTS = [
     "luna_b200_plan_linop", "luna_b200_modal_plan_create", "luna_b200_modal_plan_destroy",
     "luna_b200_modal_rhs", "luna_b200_modal_rhs_device", "luna_b200_modal_solve",
     "luna_b200_batch_set_replay", "luna_b200_batch_set_shapes", "luna_b200_radial_set_gradient",
-    "luna_b200_radial_linop",
+    "luna_b200_radial_linop", "luna_b200_modal_set_wait",
 ]
 
 _lib = None
@@ -168,6 +168,7 @@ def load():
     lib.luna_b200_modal_plan_destroy.restype = None
     lib.luna_b200_modal_rhs.argtypes = [c_void_p, PD, PD, c_double, POINTER(c_int)]
     lib.luna_b200_modal_rhs_device.argtypes = [c_void_p, c_void_p, c_void_p, c_double, c_void_p]
+    lib.luna_b200_modal_set_wait.argtypes = [c_void_p, ctypes.c_uint]
     lib.luna_b200_modal_solve.argtypes = [c_void_p, PD, PD, c_double, c_double, c_double,
                                           POINTER(SolveOpts), PD, PD, POINTER(SolveStats)]
     lib.luna_b200_batch_info.argtypes = [c_void_p, POINTER(c_int), POINTER(c_int), POINTER(c_int)]

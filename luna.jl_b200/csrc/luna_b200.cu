@@ -2366,6 +2366,7 @@ struct luna_modal_plan {
     int R = 0, C = 0;        // modal_dist_kernel: CTAs of a cluster (0: the kernels of one CTA) and clusters
     bool elem = false;       // Kerr responses alone
     ModalBar* bar = nullptr;
+    unsigned spin = 1u << 24;
     bool vplasma = false;
     ModalState* ms = nullptr;
     int* d_flags = nullptr;
@@ -2396,6 +2397,7 @@ ModalArgs modal_args(const luna_modal_plan* p, const RadState* st) {
     a.G = p->G;
     a.ms = p->ms;
     a.st = st;
+    a.spin = p->spin;
     return a;
 }
 
@@ -2653,6 +2655,12 @@ int luna_b200_modal_rhs(luna_modal_plan* p, double* nl, const double* Ew, double
     if (nevals) *nevals = nev;
     if (fl & (1 << ST_WAIT_TIMEOUT)) return fail(LUNA_WAIT_TIMEOUT, "modal_rhs: the wait of a cluster for the others timed out");
     if (fl & (1 << ST_FIELD_ABOVE_EMAX)) return fail(LUNA_FIELD_ABOVE_EMAX, "Field strength exceeds maximum for PPT ionisation rate.");
+    return LUNA_OK;
+}
+
+int luna_b200_modal_set_wait(luna_modal_plan* p, unsigned rounds) {
+    if (!p) return fail(LUNA_ERR_BAD_ARG, "modal_set_wait: null plan");
+    p->spin = rounds;
     return LUNA_OK;
 }
 

@@ -54,6 +54,7 @@ struct ModalArgs {
     void* G;                // [nslots][nmodes][M] projected polarisation per node
     ModalState* ms;
     const RadState* st;     // loop state of a solve (null for a plain evaluation)
+    unsigned spin;          // rounds after which a cluster stops waiting for the others
 };
 
 __device__ __forceinline__ bool modal_skip(const ModalArgs& a) {
@@ -436,10 +437,10 @@ struct ModalBar {
     unsigned count, gen;
 };
 
-// Barrier of all clusters of the grid (C = 1: of the cluster). False when the wait ran out; every
-// thread of a cluster returns the same.
+// Barrier of all clusters of the grid (C = 1: of the cluster). False when the wait of `spin` rounds ran
+// out; every thread of a cluster returns the same.
 template <int R>
-__device__ __forceinline__ bool modal_gsync(DWs<double>& d, ModalBar* bar, int C) {
+__device__ __forceinline__ bool modal_gsync(DWs<double>& d, ModalBar* bar, int C, unsigned spin) {
     dsync();
     if (C == 1) return true;
     if (d.rank == 0 && threadIdx.x == 0) {
@@ -453,8 +454,9 @@ __device__ __forceinline__ bool modal_gsync(DWs<double>& d, ModalBar* bar, int C
             *vg = g + 1;
         } else {
             unsigned n = 0;
-            while (*vg == g && ++n < (1u << 24)) __nanosleep(20);
-            ok = n < (1u << 24);
+            if (spin)
+                while (*vg == g && ++n < spin) __nanosleep(20);
+            ok = n < spin;
         }
         __threadfence();
         d.xs[15] = ok ? 1.0 : 0.0;
@@ -519,7 +521,7 @@ modal_dist_kernel(const LunaInst* inst, const double2* A, ModalArgs a, double2* 
             dist_c2r<double, R>(d, No / 2, Nw, [&](int k) { return E[k]; });
         for (int n = tid; n < Mb; n += T) Et[(size_t)m * Mt + base + n] = d.tb[Swz<double>::f(n)];
     }
-    bool ok = modal_gsync<R>(d, bar, C);
+    bool ok = modal_gsync<R>(d, bar, C, a.spin);
     for (int l = 0; ok; ++l) {
         const int ns = (2 << l) - 1;  // interior nodes of level l
         if (!elem) {
@@ -540,7 +542,7 @@ modal_dist_kernel(const LunaInst* inst, const double2* A, ModalArgs a, double2* 
                 }
                 dsync();  // the blocks may be written again
             }
-            if (!(ok = modal_gsync<R>(d, bar, C))) break;
+            if (!(ok = modal_gsync<R>(d, bar, C, a.spin))) break;
         }
         const double* wl = a.wts + (size_t)l * a.nslots;
         // level 0 has one node: one transform gives its rule and the midpoint rule's value
@@ -635,7 +637,7 @@ modal_dist_kernel(const LunaInst* inst, const double2* A, ModalArgs a, double2* 
                 }
             }
         }
-        if (C > 1 && !(ok = modal_gsync<R>(d, bar, C))) break;
+        if (C > 1 && !(ok = modal_gsync<R>(d, bar, C, a.spin))) break;
         if (tid == 0) {  // every CTA adds the same sums in the same order: identical decisions
             if (C > 1) {
                 e2 = v2 = 0;
@@ -655,13 +657,13 @@ modal_dist_kernel(const LunaInst* inst, const double2* A, ModalArgs a, double2* 
         if (s_done) break;
     }
     if (!ok && tid == 0) atomicOr(flags, 1 << ST_WAIT_TIMEOUT);
-    if (ok && dst) {
+    if (dst) {  // a cluster whose wait ran out leaves NaN in its modes (a call on a stream has no other answer)
         __syncthreads();
         for (int c = cl; c < nm; c += C)
             for (int k = p + R * tid; k < Nw; k += R * T) {
                 const size_t e = (size_t)c * Nw + k;
                 const cpx<double> X = reinterpret_cast<const cpx<double>*>(B)[e] * ldg(reinterpret_cast<const cpx<double>*>(a.outfac) + e);
-                dst[e] = make_double2(X.x, X.y);
+                dst[e] = ok ? make_double2(X.x, X.y) : make_double2(nan(""), nan(""));
             }
     }
     if (tid == 0 && *d.flag) atomicOr(flags, *d.flag);
