@@ -170,6 +170,9 @@ void luna_b200_plan_destroy(luna_plan* plan);
 int luna_b200_rhs(luna_plan* plan, double* nl, const double* Ew, double z);
 /* Same with device pointers, enqueued on `stream` (a cudaStream_t, may be NULL). */
 int luna_b200_rhs_device(luna_plan* plan, double* nl_dev, const double* Ew_dev, double z, void* stream);
+/* CTAs that one right-hand side of the plan takes in these two: 1, or in full precision without a
+ * pressure gradient a cluster of 4, 8 or 16. */
+int luna_b200_plan_rhs_ctas(const luna_plan* plan);
 
 /* ---------------------------------------------------------------- pressure gradients, tapers
  * A gas fill whose pressure varies along the fibre, Capillary.gradient(gas, L, p0, p1) or

@@ -110,7 +110,7 @@ EXPORTS = [
     "luna_b200_plan_linop", "luna_b200_modal_plan_create", "luna_b200_modal_plan_destroy",
     "luna_b200_modal_rhs", "luna_b200_modal_rhs_device", "luna_b200_modal_solve",
     "luna_b200_batch_set_replay", "luna_b200_batch_set_shapes", "luna_b200_radial_set_gradient",
-    "luna_b200_radial_linop", "luna_b200_modal_set_wait",
+    "luna_b200_radial_linop", "luna_b200_modal_set_wait", "luna_b200_plan_rhs_ctas",
 ]
 
 _lib = None
@@ -137,6 +137,7 @@ def load():
     lib.luna_b200_plan_destroy.argtypes = [c_void_p]
     lib.luna_b200_plan_destroy.restype = None
     lib.luna_b200_rhs.argtypes = [c_void_p, PD, PD, c_double]
+    lib.luna_b200_plan_rhs_ctas.argtypes = [c_void_p]
     lib.luna_b200_rhs_device.argtypes = [c_void_p, c_void_p, c_void_p, c_double, c_void_p]
     lib.luna_b200_solve.argtypes = [c_void_p, PD, PD, c_double, c_double, c_double,
                                     POINTER(SolveOpts), PD, PD, POINTER(SolveStats)]

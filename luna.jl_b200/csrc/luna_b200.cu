@@ -593,7 +593,7 @@ struct luna_plan {
     double2* d_nl = nullptr;
     int* d_status = nullptr;
     cudaStream_t stream = nullptr;
-    int rhs_R = 0;               // CTAs of a right-hand side (0: not decided yet)
+    int rhs_R = 1;               // CTAs of a right-hand side without a gradient
 };
 
 struct luna_batch {
@@ -824,6 +824,26 @@ bool dist_fits(const LunaInst& I, int R) {
     const int least = (sizeof(Rl) == 8 ? 1 : 2) * LUNA_BLOCK;
     return len % R == 0 && len / R >= least && len / R <= FftEmax<Rl>::v * LUNA_BLOCK && Mc % R == 0 && Mc / R >= 64 &&
            Mc <= len && I.Nw <= Mc + 1 && dist_smem_bytes(len, sizeof(cpx<Rl>), R) <= (size_t)max_smem_optin();
+}
+
+// CTAs of one FP64 right-hand side: the largest cluster that leaves each CTA a sample or sample pair a
+// thread (one launch has the GPU to itself, and what bounds it is the length of a CTA's loops); 1
+// where the distributed form does not apply. Whether clusters of a size fit is asked once per device.
+template <int R>
+bool rhs_dist_fits(const LunaInst& I) {
+    if (!dist_fits<double>(I, R)) return false;
+    static std::mutex m;
+    static std::map<std::pair<int, int>, bool> known;  // (device, bytes)
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const int sm = (int)dist_smem_bytes(dist_len(I), sizeof(cpx<double>), R);
+    std::lock_guard<std::mutex> lk(m);
+    auto it = known.find({dev, sm});
+    if (it == known.end()) it = known.insert({{dev, sm}, max_clusters(rhs_kernel_dist<R>, R, sm) > 0}).first;
+    return it->second;
+}
+int rhs_cluster(const LunaInst& I) {
+    return rhs_dist_fits<16>(I) ? 16 : rhs_dist_fits<8>(I) ? 8 : rhs_dist_fits<4>(I) ? 4 : 1;
 }
 
 // Which instances of a batch run distributed, from per-instance work estimates (single-CTA time in
@@ -1175,6 +1195,7 @@ int luna_b200_plan_create(const luna_grid_desc* g, const luna_resp_desc* resps, 
         }
     }
 #undef UP
+    if (precision == LUNA_PREC_FP64) p->rhs_R = rhs_cluster(I);
     DevPool::get().hold();
     *out = p;
     return LUNA_OK;
@@ -1186,19 +1207,6 @@ void luna_b200_plan_destroy(luna_plan* p) {
     free_all(p->allocs);
     delete p;
     DevPool::get().drop();
-}
-
-// CTAs of one FP64 right-hand side: the largest cluster that leaves each CTA 512 samples or sample
-// pairs (one launch has the GPU to itself, and what bounds it is the length of a CTA's loops); 1
-// where the distributed form does not apply.
-static int rhs_cluster(const LunaInst& I) {
-    LunaInst c = I;
-    c.grad = nullptr;  // a gradient may come and go: checked at each launch
-    auto sm = [&](int R) { return (int)dist_smem_bytes(dist_len(c), sizeof(cpx<double>), R); };
-    if (dist_fits<double>(c, 16) && max_clusters(rhs_kernel_dist<16>, 16, sm(16)) > 0) return 16;
-    if (dist_fits<double>(c, 8) && max_clusters(rhs_kernel_dist<8>, 8, sm(8)) > 0) return 8;
-    if (dist_fits<double>(c, 4) && max_clusters(rhs_kernel_dist<4>, 4, sm(4)) > 0) return 4;
-    return 1;
 }
 
 extern "C++" {
@@ -1222,13 +1230,15 @@ int launch_rhs_dist(luna_plan* p, const double2* Ew, double2* nl, cudaStream_t s
 }
 }  // extern "C++"
 
+static int rhs_ctas(const luna_plan* p) { return p->proto.grad ? 1 : p->rhs_R; }
+
 static int launch_rhs(luna_plan* p, const double2* Ew, double2* nl, cudaStream_t st, double z) {
     TwDev tw;
     int rc = get_tw(tw);
     if (rc) return rc;
     if (!p->d_inst || p->inst_stale) {
         LunaInst I = p->proto;
-        if (!p->d_gscr) {
+        if (!p->d_gscr && rhs_ctas(p) == 1) {
             size_t gb = (p->precision == LUNA_PREC_FP64) ? gscr_bytes<double>(I) : gscr_bytes<float>(I);
             if (dalloc(p->allocs, &p->d_gscr, gb)) return LUNA_ERR_CUDA;
         }
@@ -1244,12 +1254,10 @@ static int launch_rhs(luna_plan* p, const double2* Ew, double2* nl, cudaStream_t
     }
     const int maxs = max_smem_optin();
     if (p->precision == LUNA_PREC_FP64) {
-        if (!p->rhs_R) p->rhs_R = rhs_cluster(p->proto);
-        if (p->rhs_R > 1 && !p->proto.grad) {
-            const int R = p->rhs_R;
+        const int R = rhs_ctas(p);
+        if (R > 1)
             return R == 16 ? launch_rhs_dist<16>(p, Ew, nl, st, tw) : R == 8 ? launch_rhs_dist<8>(p, Ew, nl, st, tw)
                                                                              : launch_rhs_dist<4>(p, Ew, nl, st, tw);
-        }
         int sm = (int)std::min<size_t>(smem_wanted<double>(p->proto), (size_t)maxs);
         CK(allow_smem(rhs_kernel<double>));
         rhs_kernel<double><<<1, LUNA_BLOCK, sm, st>>>(p->d_inst, Ew, nl, tw.d, sm, p->d_status, z);
@@ -1374,6 +1382,8 @@ int luna_b200_plan_linop(luna_plan* p, double z, double* linop, double* outfac) 
     if (e != cudaSuccess) return fail(LUNA_ERR_CUDA, std::string("plan_linop: ") + cudaGetErrorString(e));
     return LUNA_OK;
 }
+
+int luna_b200_plan_rhs_ctas(const luna_plan* p) { return p ? rhs_ctas(p) : 0; }
 
 int luna_b200_rhs_device(luna_plan* p, double* nl_dev, const double* Ew_dev, double z, void* stream) {
     if (!p || !nl_dev || !Ew_dev) return fail(LUNA_ERR_BAD_ARG, "rhs_device: null argument");
