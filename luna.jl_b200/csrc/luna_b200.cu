@@ -569,12 +569,16 @@ size_t smem_wanted(const LunaInst& I) {
 
 }  // namespace
 
-// Device memory of one object; kept: from the pool and back to it, all work on it on streams of the
-// owner's and every copy into it on `stream`.
+// Device memory of one object, from the pool. `stream`: the one that the owner copies on and whose end is
+// that of all work on the memory when it is given back (batches and solves: theirs, plans: the legacy
+// stream); `lent`: a caller had work on another stream, whose end nothing here can wait for.
 struct DevMem {
     std::vector<void*> list;
-    bool kept = false;
-    cudaStream_t stream = nullptr;
+    cudaStream_t stream = cudaStreamLegacy;
+    bool lent = false;
+    void used_on(cudaStream_t s) {
+        if (s && s != cudaStreamLegacy) lent = true;
+    }
 };
 
 struct luna_plan {
@@ -639,13 +643,15 @@ struct luna_batch {
 
 namespace {
 
-// Device memory of batches and solves. Blocks that one gives back are kept for the next: a solve on a
-// plan that stays takes 20 to 30 buffers, and allocating and freeing them was 1.7 ms of an 11 ms
-// propagation and 3.5 ms of a 10 ms radial one. Kept are at most POOL_KEEP bytes in blocks of at most
-// POOL_BLOCK, and nothing once the last plan and batch are gone (or when an allocation fails). The
-// owner's work is on streams of its own, so giving back waits for these alone: not for the device,
-// which would hold up a caller behind other threads' work and is an error while any stream is captured.
-// The lock covers the books, not what waits. Blocks are cleared like fresh ones.
+// Device memory of plans, batches and solves. Blocks that an object gives back are kept for the next one:
+// a solve on a plan that stays takes 20 to 30 buffers, and allocating and freeing them was 1.7 ms of an
+// 11 ms propagation and 3.5 ms of a 10 ms radial one; creating and destroying a plan with a rate table
+// takes 1.4 ms without and 0.4 ms with it. Kept are at most POOL_KEEP bytes in blocks of at most
+// POOL_BLOCK, and nothing once the last plan and batch are gone (or when an allocation fails). Giving back
+// waits for the object's stream alone: not for the device, which would hold up a caller behind other
+// threads' work and is an error while any stream is captured. Memory lent to a caller's stream is freed
+// (cudaFree does the waiting), as is a plan's while the legacy stream is drawn into a capture. The lock
+// covers the books, not what waits. Blocks are cleared like fresh ones.
 struct DevPool {
     static constexpr size_t POOL_KEEP = (size_t)64 << 20, POOL_BLOCK = (size_t)16 << 20;
     struct Block {
@@ -717,17 +723,20 @@ struct DevPool {
         }
         return e;
     }
-    // s: the owner's stream, the only one with work on the blocks
-    void give(std::vector<void*>& list, cudaStream_t s) {
-        if (list.empty()) return;
+    void give(const DevMem& mem) {
+        const cudaStream_t s = mem.stream;
+        if (mem.list.empty()) return;
         int dev = 0;
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         // (a device in an error state keeps nothing)
-        bool keep = s && cudaStreamSynchronize(s) == cudaSuccess && cudaGetDevice(&dev) == cudaSuccess;
+        bool keep = !mem.lent && cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
+                           cudaStreamSynchronize(s) == cudaSuccess && cudaGetDevice(&dev) == cudaSuccess;
+        if (!keep) cudaGetLastError();
         std::vector<std::pair<size_t, void*>> kept;
         std::vector<void*> out;
         {
             std::lock_guard<std::mutex> lk(m);
-            for (void* p : list) {
+            for (void* p : mem.list) {
                 auto it = live.find(p);
                 const Block b = it->second;
                 live.erase(it);
@@ -760,16 +769,16 @@ template <typename T>
 int dalloc(DevMem& m, T** p, size_t bytes) {
     void* q = nullptr;
     if (bytes < 1) bytes = 16;
-    CK(m.kept ? DevPool::get().take(&q, bytes) : cudaMalloc(&q, bytes));
+    CK(DevPool::get().take(&q, bytes));
     m.list.push_back(q);
     *p = reinterpret_cast<T*>(q);
     return LUNA_OK;
 }
 
-// host array into the object's memory: complete on return, or (kept memory) in the order of its stream
+// host array into the object's memory, in the order of its stream
 template <typename T>
 int h2d(DevMem& m, T* dst, const void* src, size_t bytes) {
-    if (m.kept) CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, m.stream));
+    if (m.stream != cudaStreamLegacy) CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, m.stream));
     else CK(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
     return LUNA_OK;
 }
@@ -784,9 +793,7 @@ int upload(DevMem& m, const T* src, size_t n, const T** dst) {
 }
 
 void free_all(DevMem& m) {
-    if (m.kept) DevPool::get().give(m.list, m.stream);
-    else
-        for (void* p : m.list) cudaFree(p);
+    DevPool::get().give(m);
     m.list.clear();
 }
 
@@ -1203,13 +1210,29 @@ int luna_b200_plan_create(const luna_grid_desc* g, const luna_resp_desc* resps, 
 
 void luna_b200_plan_destroy(luna_plan* p) {
     if (!p) return;
-    if (p->stream) cudaStreamDestroy(p->stream);
+    if (p->stream) {
+        cudaStreamSynchronize(p->stream);
+        cudaStreamDestroy(p->stream);
+    }
     free_all(p->allocs);
     delete p;
     DevPool::get().drop();
 }
 
 extern "C++" {
+// a radial or modal plan with its column plan, whose tables its kernels read
+template <typename PlanT>
+void column_plan_free(PlanT* p) {
+    if (p->stream) {
+        cudaStreamSynchronize(p->stream);
+        cudaStreamDestroy(p->stream);
+    }
+    p->col->allocs.lent = p->col->allocs.lent || p->allocs.lent;
+    free_all(p->allocs);
+    luna_b200_plan_destroy(p->col);
+    delete p;
+}
+
 template <int R>
 int launch_rhs_dist(luna_plan* p, const double2* Ew, double2* nl, cudaStream_t st, const TwDev& tw) {
     const int sm = (int)dist_smem_bytes(dist_len(p->proto), sizeof(cpx<double>), R);
@@ -1236,6 +1259,7 @@ static int launch_rhs(luna_plan* p, const double2* Ew, double2* nl, cudaStream_t
     TwDev tw;
     int rc = get_tw(tw);
     if (rc) return rc;
+    if (st != p->stream) p->allocs.used_on(st);
     if (!p->d_inst || p->inst_stale) {
         LunaInst I = p->proto;
         if (!p->d_gscr && rhs_ctas(p) == 1) {
@@ -1442,7 +1466,6 @@ int luna_b200_batch_create(luna_plan* const* plans, int n, const luna_solve_opts
         cudaEventCreateWithFlags(&b->evj, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->evj3, cudaEventDisableTiming) != cudaSuccess)
         return bail(fail(LUNA_ERR_CUDA, "batch_create: stream/event creation failed"));
-    b->allocs.kept = true;
     b->allocs.stream = b->stream;
     if (opts->saveN > 0) {
         const double* zs = nullptr;
@@ -1590,6 +1613,8 @@ int luna_b200_batch_create(luna_plan* const* plans, int n, const luna_solve_opts
             }
         }
     }
+    if (cudaStreamSynchronize(b->stream) != cudaSuccess)  // the caller's arrays have been read
+        return bail(fail(LUNA_ERR_CUDA, "batch_create: copying failed"));
     *out = b;
     return LUNA_OK;
 }
@@ -1635,8 +1660,7 @@ int luna_b200_batch_upload(luna_batch* b, const double* const* linops, const dou
     return LUNA_OK;
 }
 
-int luna_b200_batch_run(luna_batch* b, float* device_ms) {
-    if (!b) return fail(LUNA_ERR_BAD_ARG, "batch_run: null batch");
+static int batch_run(luna_batch* b, float* device_ms) {
     TwDev tw;
     int rc = get_tw(tw);
     if (rc) return rc;
@@ -1686,6 +1710,14 @@ int luna_b200_batch_run(luna_batch* b, float* device_ms) {
     CK(cudaEventSynchronize(b->ev1));
     if (device_ms) CK(cudaEventElapsedTime(device_ms, b->ev0, b->ev1));
     return LUNA_OK;
+}
+
+int luna_b200_batch_run(luna_batch* b, float* device_ms) {
+    if (!b) return fail(LUNA_ERR_BAD_ARG, "batch_run: null batch");
+    const int rc = batch_run(b, device_ms);
+    if (rc)  // no work is left behind: the plans' memory may be given back
+        for (cudaStream_t s : {b->stream3, b->stream2, b->stream}) cudaStreamSynchronize(s);
+    return rc;
 }
 
 int luna_b200_batch_download(luna_batch* b, double* const* saves, double* const* y_out, luna_solve_stats* stats) {
@@ -1798,6 +1830,7 @@ int luna_b200_batch_set_replay(luna_batch* b, int i, const double* replay, long 
     }
     const double* rp = nullptr;
     if (upload(b->allocs, replay, 2 * (size_t)nreplay, &rp)) return LUNA_ERR_CUDA;
+    CK(cudaStreamSynchronize(b->stream));  // the caller's array has been read
     I.replay = rp;
     I.nreplay = nreplay;
     return LUNA_OK;
@@ -1805,9 +1838,6 @@ int luna_b200_batch_set_replay(luna_batch* b, int i, const double* replay, long 
 
 void luna_b200_batch_destroy(luna_batch* b) {
     if (!b) return;
-    // a run that ended in an error may have left work behind
-    if (b->stream3) cudaStreamSynchronize(b->stream3);
-    if (b->stream2) cudaStreamSynchronize(b->stream2);
     free_all(b->allocs);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
@@ -2065,16 +2095,14 @@ int luna_b200_radial_plan_create(const luna_grid_desc* g, const luna_resp_desc* 
 
 void luna_b200_radial_plan_destroy(luna_radial_plan* p) {
     if (!p) return;
-    if (p->stream) cudaStreamDestroy(p->stream);
     if (p->h_fin) cudaFreeHost(p->h_fin);
-    free_all(p->allocs);
-    luna_b200_plan_destroy(p->col);
-    delete p;
+    column_plan_free(p);
 }
 
 int luna_b200_radial_rhs_device(luna_radial_plan* p, double* nl_dev, const double* Ew_dev, double z, void* stream) {
     (void)z;  // constant density and normalisation
     if (!p || !nl_dev || !Ew_dev) return fail(LUNA_ERR_BAD_ARG, "radial_rhs_device: null argument");
+    p->allocs.used_on((cudaStream_t)stream);
     if (p->precision == LUNA_PREC_FP64) return rad_rhs<double>(p, (const double2*)Ew_dev, (double2*)nl_dev, (cudaStream_t)stream, z);
     return rad_rhs<float>(p, (const double2*)Ew_dev, (double2*)nl_dev, (cudaStream_t)stream, z);
 }
@@ -2157,6 +2185,7 @@ int luna_b200_qdht_device(luna_radial_plan* p, void* Y_dev, const void* X_dev, i
     if (!p || !Y_dev || !X_dev || X_dev == Y_dev) return fail(LUNA_ERR_BAD_ARG, "qdht_device: null or aliased argument");
     if (((uintptr_t)X_dev | (uintptr_t)Y_dev) & 7)
         return fail(LUNA_ERR_BAD_ARG, "qdht_device: X and Y must be 8-byte aligned");
+    p->allocs.used_on((cudaStream_t)stream);
     rad_qdht(p, X_dev, forward != 0, Y_dev, nullptr, p->d_flags, (cudaStream_t)stream);
     CK(cudaGetLastError());
     return LUNA_OK;
@@ -2220,7 +2249,6 @@ int col_solve(PlanT* p, XF&& xform, const char* who, const double* linop, double
     if (!p->stream) CK(cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking));
     const cudaStream_t s = p->stream;
     RadSolve S;
-    S.allocs.kept = true;
     S.allocs.stream = s;
     if (G.g && dalloc(S.allocs, &S.ofz, cb * n)) return LUNA_ERR_CUDA;
     if (dalloc(S.allocs, &S.L, cb * n) || dalloc(S.allocs, &S.y, cb * n) || dalloc(S.allocs, &S.yn, cb * n) ||
@@ -2631,16 +2659,14 @@ int luna_b200_modal_plan_create(const luna_grid_desc* g, const luna_resp_desc* r
 
 void luna_b200_modal_plan_destroy(luna_modal_plan* p) {
     if (!p) return;
-    if (p->stream) cudaStreamDestroy(p->stream);
     if (p->h_fin) cudaFreeHost(p->h_fin);
-    free_all(p->allocs);
-    luna_b200_plan_destroy(p->col);
-    delete p;
+    column_plan_free(p);
 }
 
 int luna_b200_modal_rhs_device(luna_modal_plan* p, double* nl_dev, const double* Ew_dev, double z, void* stream) {
     (void)z;  // constant density
     if (!p || !nl_dev || !Ew_dev) return fail(LUNA_ERR_BAD_ARG, "modal_rhs_device: null argument");
+    p->allocs.used_on((cudaStream_t)stream);
     if (p->precision == LUNA_PREC_FP64) return modal_rhs<double>(p, (const double2*)Ew_dev, (double2*)nl_dev, (cudaStream_t)stream);
     return modal_rhs<float>(p, (const double2*)Ew_dev, (double2*)nl_dev, (cudaStream_t)stream);
 }
@@ -2772,6 +2798,7 @@ extern "C" int luna_b200_rhs_device_noalloc(luna_plan* p, double* nl_dev, const 
     rc = find_tw(tw);
     if (rc) return rc;
     I.gscr = scratch;
+    p->allocs.used_on((cudaStream_t)stream);
     const int maxs = max_smem_optin();
     cudaStream_t st = (cudaStream_t)stream;
     if (p->precision == LUNA_PREC_FP64) {
