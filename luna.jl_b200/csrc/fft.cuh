@@ -288,6 +288,12 @@ __device__ __forceinline__ void sub_fft_s(unsigned off, int Mb, const TwTab<R>& 
     if constexpr (E > 4) { if (rem == 2) pass_s<R, INV, E, 4>(off, Mb, 1, t, tw); }
     for (int L = 1 << rem; L < Mb; L *= E) pass_s<R, INV, E, E>(off, Mb, L, t, tw);
 }
+// Radix-2 passes (FP32 sub-transforms of up to 1024 points) in one function: a pass is a single
+// butterfly a thread, and nine or ten calls were a tenth of a right-hand side.
+template <typename R, bool INV>
+__device__ __noinline__ void sub_fft_r2(unsigned off, int Mb, int t, const TwTab<R> tw) {
+    sub_fft<R, INV, 2>(dsm_ptr<R>(off), Mb, tw, t);
+}
 template <typename R, bool INV, int P>
 __device__ __noinline__ void join_pass_s(unsigned off, int M, const TwTab<R> tw) {
     join_pass<R, INV, P>(dsm_ptr<R>(off), M, tw);
@@ -323,7 +329,7 @@ __device__ __forceinline__ void sub_ffts(unsigned off, int M, int P, const TwTab
     for (int p = 0; p < P; ++p, off += (unsigned)(Mb * sizeof(cpx<R>))) {
         if (E == 8) sub_fft_s<R, INV, 8>(off, Mb, tw, threadIdx.x);
         else if (E == 4) sub_fft_s<R, INV, 4>(off, Mb, tw, threadIdx.x);
-        else sub_fft_s<R, INV, 2>(off, Mb, tw, threadIdx.x);
+        else sub_fft_r2<R, INV>(off, Mb, threadIdx.x, tw);
     }
 }
 

@@ -9,6 +9,7 @@ import pytest
 from luna_b200 import _lib
 from luna_b200 import plan as P
 from luna_b200.interface import prop_capillary_args, prop_gnlse_args
+from oracle import uppe
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +53,16 @@ def test_solves_from_the_smallest_grids_that_go_to_clusters(make, precision, on)
     for flags, expect in ((0, on), (_lib.SOLVE_NO_DIST | _lib.SOLVE_NO_CLUSTERS, 0)):
         b = P.Batch([P.Plan.from_transform(p.transform, precision)], 2, np.array([0.0, p.grid.zmax]), flags=flags)
         assert b.info()[1:] == (expect, expect)
+
+
+@pytest.mark.parametrize("make,No", [(lambda: _capillary(0.06e-12), 1024), (lambda: _capillary(0.12e-12, gas="H2"), 2048),
+                                     (lambda: _capillary(0.25e-12), 4096), (lambda: _gnlse(1e-12), 1024)])
+def test_smallest_mixed_right_hand_sides(make, No):
+    """Sub-transforms of 512 and 1024 points in radix-2 passes, the next size in radix 4; the bound is the
+    parity tests' for mixed precision."""
+    p = make()
+    assert p.grid.No == No
+    E = p.Eω * np.exp(1j * 0.2 * np.random.default_rng(5).standard_normal(len(p.Eω)))
+    nl = P.Plan.from_transform(p.transform, _lib.PREC_MIXED).rhs(np.zeros_like(E), E)
+    ref = uppe.trans_mode_avg(p.transform, E, 0.0)
+    assert np.linalg.norm(nl - ref) <= 1e-5 * np.linalg.norm(ref)
