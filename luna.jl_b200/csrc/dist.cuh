@@ -567,10 +567,11 @@ struct RateF {
 // of the CTAs before it) and the integrands' first samples exchanged through the cluster.
 // Mixed precision: rates, ionisation fractions (1 - exp(-x) as -expm1(-x)) and the
 // ionisation-loss current are FP32 per sample (kept in shared memory at [s*T + tid]
-// between the passes), the running integrals FP64. FP64: every quantity FP64.
+// between the passes), the running integrals FP64.
 template <typename Rl, int NS, int R>
 __device__ __noinline__ void dist_plasma(const LunaInst& I, DWs<Rl>& d, int M, double sc, int ip, int ir, double kc,
                                          double rc) {
+    static_assert(sizeof(Rl) == 4, "full precision: dist_plasma_f64");
     const int q = d.rank, T = LUNA_BLOCK, tid = threadIdx.x;
     const int Mb = M / R;
     const int mbase = q * Mb;
@@ -578,9 +579,6 @@ __device__ __noinline__ void dist_plasma(const LunaInst& I, DWs<Rl>& d, int M, d
     const double dt = r.dt, er = r.eratio, preion = r.preion, coef = r.coef;
     const float ipf = (float)r.ionpot;
     const int pr0 = tid * (NS / 2);
-    // per-sample rates and ionisation fractions in the solver's precision: FP32 in mixed
-    // precision, FP64 (the arithmetic of the single-CTA FP64 plasma scan) otherwise
-    constexpr bool F64 = sizeof(Rl) == 8;
     Rl* rrb = reinterpret_cast<Rl*>(d.stg);  // rates (the staged spectrum is dead)
     Rl* frb = reinterpret_cast<Rl*>(d.fb);   // ionisation fractions
     Rl ev[NS];  // stored field samples; E = ev * sc
@@ -594,17 +592,7 @@ __device__ __noinline__ void dist_plasma(const LunaInst& I, DWs<Rl>& d, int M, d
     // pass A: rates; exclusive scan of the thread sums and the block total
     double racc = 0;
     Rl r0 = 0;
-    if constexpr (F64) {
-        const bool ppt = r.kind == LUNA_RESP_PLASMA_PPT;
-#pragma unroll
-        for (int s = 0; s < NS; ++s) {
-            const double aE = fabs(E(s));
-            const double rv = ppt ? ppt_rate<double>(r, aE, d.flag) : adk_rate<double>(r, aE);
-            rrb[s * T + tid] = rv;
-            racc += rv;
-            if (s == 0) r0 = rv;
-        }
-    } else {
+    {
         RateF rf;
         rf.init(r);
 #pragma unroll
@@ -638,14 +626,8 @@ __device__ __noinline__ void dist_plasma(const LunaInst& I, DWs<Rl>& d, int M, d
         for (int s = 0; s < NS; ++s) {
             const double rr = rrb[s * T + tid];
             S += rr;
-            Rl fr;
-            if constexpr (F64) {
-                const double f = dt * (S - 0.5 * (y0r + rr));
-                fr = preion + 1.0 - ((f == 0.0) ? 1.0 : exp(-f));
-            } else {
-                const float fx = (float)(dt * (S - 0.5 * (y0r + rr)));
-                fr = (float)(preion - (double)expm1f(-fx));
-            }
+            const float fx = (float)(dt * (S - 0.5 * (y0r + rr)));
+            const Rl fr = (float)(preion - (double)expm1f(-fx));
             frb[s * T + tid] = fr;
             const double ph = (double)fr * er * E(s);
             ph_acc += ph;
@@ -666,14 +648,8 @@ __device__ __noinline__ void dist_plasma(const LunaInst& I, DWs<Rl>& d, int M, d
         const Rl rr = rrb[s * T + tid], fr = frb[s * T + tid];
         const double ph = (double)fr * er * E(s);
         Tv += ph;
-        double ion;
-        if constexpr (F64) {
-            const double Es = E(s);
-            ion = (fabs(Es) > 0) ? r.ionpot * rr * (1.0 - fr) / Es : 0.0;
-        } else {
-            const float Ef = (float)E(s);
-            ion = (double)((Ef != 0.0f) ? ipf * rr * (1.0f - fr) / Ef : 0.0f);
-        }
+        const float Ef = (float)E(s);
+        const double ion = (double)((Ef != 0.0f) ? ipf * rr * (1.0f - fr) / Ef : 0.0f);
         return dt * (Tv - 0.5 * (y0p + ph)) + ion;
     };
     double J_acc = 0, J_first = 0;
@@ -723,8 +699,8 @@ __device__ __noinline__ void dist_plasma(const LunaInst& I, DWs<Rl>& d, int M, d
 
 // The FP64 form: NS consecutive samples of this CTA's block per thread, every quantity FP64, the
 // exchange of carries and first samples as in dist_plasma. The samples' rates, fractions and
-// currents stay in registers up to eight a thread (dist_plasma's passes over shared memory took
-// 1.2-1.8 kB of spill traffic in FP64) and the rates are evaluated together (rates_f64); a warp
+// currents stay in registers up to eight a thread (passes over shared memory as in dist_plasma took
+// 1.2-1.8 kB of spill traffic) and the rates are evaluated together (rates_f64); a warp
 // without ionisation takes one exp for its samples and no loss current.
 template <int NS, int R>
 __device__ __noinline__ void dist_plasma_f64(const LunaInst& I, DWs<double>& d, int M, double sc, int ip, int ir,
