@@ -541,6 +541,13 @@ int get_tw(TwDev& out) {
 
 bool is_pow2(int x) { return x > 0 && (x & (x - 1)) == 0; }
 
+int sm_count() {
+    int dev = 0, v = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    return v;
+}
+
 int max_smem_optin() {
     int dev = 0, v = 0;
     cudaGetDevice(&dev);
@@ -1964,14 +1971,16 @@ void launch_pdl(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStr
 
 // Er = A Mi^T or Pk = Pw Mf^T along the radial index of the 2Nw x Nr real view: FP64
 // CUDA-core tiles for the plain path, 3xBF16 tensor-core products for the mixed path. FP64 takes
-// 64 x 64 tiles where they occupy most SMs (half of 148: above, the larger tile's fewer
-// shared-memory reads a product count), 32 x 32 below.
+// 32 x 32 tiles while all of them run at one time (three an SM), 64 x 64 above, whose fewer
+// shared-memory reads a product then count. Tile of 64 against 32 at 2 Nw x Nr, us: 514 x 64 7.2 / 3.7,
+// 2050 x 128 12.7 / 9.0, 2050 x 192 (390 tiles of 32) 18.2 / 17.7, 4098 x 128 (516) 12.9 / 21.7,
+// 2050 x 256 (520) 23.6 / 41.1, 4098 x 384 87.4 / 111.3.
 int rad_qdht(luna_radial_plan* p, const void* X, bool fwd, void* Y, const RadState* st, int* flags, cudaStream_t s) {
     const int rows = 2 * p->Nw;
     if (p->precision == LUNA_PREC_FP64) {
-        const int g64 = (rows + 63) / 64 * ((p->Nr + 63) / 64);
+        const int g32 = (rows + 31) / 32 * ((p->Nr + 31) / 32);
         const double* Mx = fwd ? p->Mf : p->Mi;
-        if (g64 >= 74)
+        if (g32 > 3 * sm_count())
             launch_pdl(rad_gemm_f64<64>, dim3((rows + 63) / 64, (p->Nr + 63) / 64), 256, 0, s, (const double*)X, rows, rows, Mx,
                        (double*)Y, p->Nr, st);
         else
@@ -2299,7 +2308,7 @@ int col_solve(PlanT* p, XF&& xform, const char* who, const double* linop, double
     const int eg = rad_grid(n);
     // FP64 without a gradient: a stage's store and the next stage's input in one launch
     const bool fused = sizeof(Rl) == 8 && !G.g;
-    const int ng = (int)std::min<size_t>((n + 127) / 128, 148 * 16);
+    const int ng = (int)std::min<size_t>((n + 127) / 128, sm_count() * 16);
     int* flags_dev = (int*)((char*)S.st + offsetof(RadState, flags));
     const int* fin_dev = (const int*)((char*)S.st + offsetof(RadState, finished));
     rad_init_kernel<<<1, 32, 0, s>>>(S.st, S.opt, S.y, S.yn, S.d_k);
@@ -2473,8 +2482,11 @@ int modal_dist(luna_modal_plan* p, const double2* src, double2* dst, const TwTab
 
 // Clusters of a plan: full precision, time buffers that give each CTA of a cluster 512
 // samples, and not the two-component plasma (its scans run on one CTA a node). As many clusters as
-// modes (Kerr alone: 72 us at No = 16384 with one mode, 332 us with the kernels of one CTA) or as nodes of
-// the third refinement, if that many are resident together.
+// modes (Kerr alone: 72 us at No = 16384 with one mode, 332 us with the kernels of one CTA; four modes at
+// No = 8192 299 us on one cluster, 111 on four, 110 on eight), with other responses eight, if that many
+// are resident together: clusters then share a level's nodes, and most levels have eight or fewer
+// (plasma, No = 16384, one mode: 537 us on one cluster, 258 on four, 244 on eight, 240 on nine; two modes
+// at 8192: 1826, 626, 438, 431; Raman, one mode: 313, 176, 163, 162).
 template <int R>
 bool modal_dist_setup(luna_modal_plan* p) {
     const LunaInst& I = p->col->proto;
