@@ -146,3 +146,75 @@ def test_statistics_with_a_warp_or_a_block_a_row(B, N, nspec, members):
     var = d.var(0, unbiased=False)[:, :nspec].amax(1) if nspec and members > 1 else torch.zeros(B, device="cuda").double()
     msq = (d ** 2).mean(0)[:, :max(nspec, 1)].amax(1)
     assert ((spread.double() ** 2 - var).abs() <= 4 * members * 2.0 ** -23 * msq).all()
+
+
+def _blocks(torch, values, bad):
+    """Columns of 32 values, the first of each block replaced by `bad` in a second copy: 31 of 32 columns
+    are the same values once in the range of the common case and once beside one outside."""
+    a = values.view(-1, 32).clone()
+    a[:, 0] = 0.5
+    b = a.clone()
+    b[:, 0] = bad
+    return a.flatten(), b.flatten()
+
+
+@pytest.mark.parametrize("bad,act", [(-70.0, 0.0), (1e31, 1e31), (float("inf"), float("inf")), (float("-inf"), float("nan")),
+                                     (float("nan"), float("nan"))])
+def test_silu_is_the_same_beside_values_out_of_its_common_range(bad, act):
+    """act(v) of biases over all exponents from 2^-126 to 2^99 and both signs (v > -69): the division
+    without a range check gives the operator's bits, and the operator's form takes what lies
+    outside. Against 64-bit values: __expf within 2 + 1.173 |v| ulp and three roundings of 2^-24."""
+    torch, lib, p, st = _sg()
+    g = torch.Generator(device="cuda").manual_seed(1)
+    n = 1 << 17
+    mant, ex = 1 + torch.rand(n, device="cuda", generator=g), torch.randint(-126, 100, (n,), device="cuda", generator=g)
+    v = torch.ldexp(mant, ex)
+    w = torch.where(torch.rand(n, device="cuda", generator=g) < 0.5, torch.ldexp(mant, ex.clamp(max=5)), 68.9 * torch.rand(n, device="cuda", generator=g))
+    v = torch.cat([v, -w.clamp(max=68.9), torch.tensor([0.0, -0.0] * 16, device="cuda"), 80 * torch.rand(n - 32, device="cuda", generator=g)])
+    B, K = 128, 64
+    X, W = torch.zeros(B, K, dtype=torch.bfloat16, device="cuda"), torch.zeros(v.numel(), K, dtype=torch.bfloat16, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = []
+    for b in _blocks(torch, v, bad):
+        Y = torch.empty(B, b.numel(), device="cuda")
+        assert lib.luna_sg_linear_fwd(p(X), 0, p(W), p(b), B, K, b.numel(), 1, None, None, p(Y), 1, p(err), st) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(Y[0].view(torch.int32), Y[-1].view(torch.int32))
+        out.append(Y[0].view(-1, 32))
+    a, b = out
+    assert int(err.item()) == 0 and torch.equal(a[:, 1:].view(torch.int32), b[:, 1:].view(torch.int32))
+    x = v.view(-1, 32)[:, 1:].double()
+    ref = x * torch.sigmoid(x)
+    tol = ((2 + 1.173 * x.abs().clamp(max=100)) * 2.0 ** -23 + 3 * 2.0 ** -24) * ref.abs() + 2.0 ** -149
+    assert ((a[:, 1:].double() - ref).abs() <= tol).all()
+    assert torch.allclose(b[:, 0].double(), torch.full_like(b[:, 0], act).double(), rtol=1e-6, atol=1e-27, equal_nan=True)
+
+
+@pytest.mark.parametrize("bad", [-70.0, 1e31, float("inf"), float("nan")])
+def test_silu_derivative_is_the_same_beside_values_out_of_its_common_range(bad):
+    """v silu'(z) for every BF16 z above -69, v = 1: a warp's rows share eight columns, so a value out of
+    range in one row sends the others through the operator's form."""
+    torch, lib, p, st = _sg()
+    bits = torch.arange(1 << 16, device="cuda", dtype=torch.int32).to(torch.int16)
+    z = bits.view(torch.bfloat16)
+    z = z[torch.isfinite(z) & (z > -69) & (z < 1e30)]
+    z = torch.cat([z, z[: (-z.numel()) % (4 * 31 * 128)]]).view(-1, 4, 31, 128)  # 31 of a warp's 32 rows
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    B, K, N = 128, 128, 128
+    dZ, W = (torch.zeros(B, N, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    dZ[:, 0] = 1
+    W[0, :] = 1  # dZ W = 1 everywhere
+    for block in z:
+        out = []
+        for q in (0.5, bad):
+            Zp = torch.cat([block, torch.full((4, 1, K), q, dtype=torch.bfloat16, device="cuda")], 1).contiguous()
+            dX = torch.empty(B, K, dtype=torch.bfloat16, device="cuda")
+            assert lib.luna_sg_linear_bwd_data(p(dZ), p(W), p(Zp), B, K, N, p(dX), 1, p(err), st) == 0
+            out.append(dX.view(4, 32, K)[:, :-1])
+        torch.cuda.synchronize()
+        assert torch.equal(out[0].view(torch.int16), out[1].view(torch.int16))
+        x = block.double()
+        s = torch.sigmoid(x)
+        ref = s * (1 + x * (1 - s))
+        assert ((out[0].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5).all()
+    assert int(err.item()) == 0
