@@ -69,3 +69,27 @@ def test_table_that_begins_at_a_zero_field(trange, monkeypatch):
     tol = 1000 * _rel(uppe.trans_mode_avg(p.transform, E, 0.0), ref)
     for rc, nl in _rhs(p.transform, E):
         assert rc == 0 and _rel(nl, ref) < tol
+
+
+@pytest.mark.parametrize("trange", TRANGES)
+def test_nan_field_gives_nan_and_field_above_the_table_is_reported(trange):
+    p = _problem(trange)
+    E = p.Eω.copy()
+    E[len(E) // 3] = np.nan
+    for rc, nl in _rhs(p.transform, E):
+        assert rc == _lib.LUNA_OK and np.all(np.isnan(nl))
+    for rc, _ in _rhs(p.transform, 50.0 * p.Eω):
+        assert rc == _lib.LUNA_FIELD_ABOVE_EMAX
+
+
+@pytest.mark.parametrize("trange", TRANGES)
+def test_adk_rates_follow_the_oracle(trange):
+    """The logarithmic form of the ADK rate against the power, from the threshold to ionisation of a
+    visible part of the gas; 1e-11 as the parity tests have it for right-hand sides with plasma."""
+    p = _problem(trange, plasma="ADK")
+    assert next(q for q in p.transform.resp if q.kind == "plasma").ratefunc.kind == "adk"
+    E = p.Eω * np.exp(1j * 0.2 * np.random.default_rng(3).standard_normal(len(p.Eω)))
+    for f in (0.3, 1.0, 2.0):
+        ref = uppe.trans_mode_avg(p.transform, f * E, 0.0)
+        for rc, nl in _rhs(p.transform, f * E):
+            assert rc == 0 and _rel(nl, ref) < 1e-11

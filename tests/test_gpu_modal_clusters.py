@@ -8,10 +8,10 @@ luna_b200_loader.load()
 import numpy as np
 import pytest
 
-from luna_b200 import _lib, fields, ionisation, modal, modes
+from luna_b200 import _lib, fields, ionisation, modal, modes, raman
 from luna_b200 import physdata as pd
 from luna_b200.grid import RealGrid
-from luna_b200.nonlinear import Kerr_field, PlasmaCumtrapz
+from luna_b200.nonlinear import Kerr_field, PlasmaCumtrapz, RamanPolarField
 from oracle import uppe
 
 pytestmark = pytest.mark.gpu
@@ -21,14 +21,16 @@ def _rel(a, b):
     return float(np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-300))
 
 
-def _case(nm, trange, plasma=False):
-    ms = tuple(modes.MarcatiliMode(50e-6, "Ar", 1.0, n=1, m=m + 1, loss=False) for m in range(nm))
+def _case(nm, trange, plasma=False, gas="Ar"):
+    ms = tuple(modes.MarcatiliMode(50e-6, gas, 1.0, n=1, m=m + 1, loss=False) for m in range(nm))
     grid = RealGrid(1e-3, 800e-9, (160e-9, 3000e-9), trange)
-    resp = [Kerr_field(pd.gamma3_gas("Ar"))]
+    resp = [Kerr_field(pd.gamma3_gas(gas))]
+    if gas == "H2":
+        resp.append(RamanPolarField(grid.to, raman.raman_response(grid.to, gas)))
     if plasma:
         resp.append(PlasmaCumtrapz(grid.to, grid.to, ionisation.ionrate_PPTaccel("Ar", 800e-9, N=2 ** 12),
                                    pd.ionisation_potential("Ar")))
-    E, t = modal.setup_modal(grid, pd.density("Ar", 1.0), resp, fields.GaussField(800e-9, 10e-15, energy=20e-6), ms, "y")
+    E, t = modal.setup_modal(grid, pd.density(gas, 1.0), resp, fields.GaussField(800e-9, 10e-15, energy=20e-6), ms, "y")
     for m in range(1, nm):
         E[:, m] = 0.3 / m * E[:, 0]
     return grid, E, t, modal.make_const_linop_modes(grid, ms, 800e-9)
@@ -57,3 +59,15 @@ def test_a_wait_that_runs_out_is_reported(nm, plasma):
     assert lib.luna_b200_modal_set_wait(plan._h, 1 << 24) == 0
     assert np.array_equal(plan.rhs(np.zeros_like(E), E), ref)
     assert plan.solve(linop, E, 0.0, 1e-5, 1e-4, saveN=2).status == 0
+
+
+@pytest.mark.parametrize("nm,trange,plasma,gas", [(3, 0.2e-12, True, "Ar"), (1, 0.1e-12, True, "Ar"), (5, 0.4e-12, True, "Ar"), (2, 0.2e-12, False, "H2"),
+                                                  (2, 1e-12, False, "H2"), (9, 0.2e-12, False, "H2")])
+def test_several_modes_with_plasma_or_raman(nm, trange, plasma, gas):
+    """Levels whose nodes the clusters share, fewer, as many and more modes than clusters, clusters of 4 to
+    16; 1e-11 as the modal tests have it with plasma or Raman."""
+    grid, E, t, _ = _case(nm, trange, plasma, gas)
+    nl = np.zeros_like(E)
+    t(nl, E, 0.0)
+    assert _rel(nl, uppe.trans_modal(t, E, 0.0)) < 1e-11
+    assert t.plan().nevals == t.oracle_nevals
