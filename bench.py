@@ -300,10 +300,10 @@ def cpu_estimate(sample_seconds=20.0, workers=1, pool=None):
 
 def plain_fp64_measured(inst, probs, dur, status64, k=8):
     """The plain FP64 drop-in, measured: one single-instance FP64 solve after another (a
-    batch of one, as luna_b200_solve runs it: on a cluster for the long grids, 16 CTAs for
-    No = 32768 and 8 for No = 16384, on one CTA otherwise), device time with CUDA events, for
-    a stratified subset of the completed instances: in each of the two strata (cluster,
-    single CTA) k quantiles of their integration times in the single-CTA FP64 batch.
+    batch of one, as luna_b200_solve runs it: on a cluster of 16 CTAs from No = 16384, of 8
+    for No = 8192), device time with CUDA events, for a stratified subset of the completed
+    instances: in each of the two strata (clusters of 16, of 8) k quantiles of their
+    integration times in the single-CTA FP64 batch.
     Returns the subset's own
     sims/hour, the scan estimate (per stratum, the batch's per-instance times scaled by the
     subset's measured/batch ratio) and the per-instance record."""
@@ -312,7 +312,7 @@ def plain_fp64_measured(inst, probs, dur, status64, k=8):
     for i in done:
         strata[probs[i].grid.No >= 16384].append(i)
     rows, t_all, n_all, scan_s = [], 0.0, 0, 0.0
-    for big, members in strata.items():
+    for members in strata.values():  # clusters of 16, of 8
         if not members:
             continue
         order = sorted(members, key=lambda i: dur[i])
@@ -1056,7 +1056,7 @@ def main():
                 plain = {"value": v_scan, "unit": "sims/hour", "subset_value": v_sub,
                          "method": ("plain FP64 drop-in measured: one single-instance FP64 solve after another "
                                     f"(device time; clusters of 16 CTAs from No = 16384, of 8 for No = 8192) for {len(rows)} instances, "
-                                    "8 quantiles of the single-CTA FP64 batch time in each of the two strata; value = "
+                                    "8 quantiles of the single-CTA FP64 batch time in each of the two strata (clusters of 16, of 8); value = "
                                     "the scan's sims/hour with each stratum's per-instance batch times scaled by its "
                                     "subset's measured/batch ratio, subset_value = the subset's own"),
                          "subset": rows, "speedup_of_value": value / v_scan}

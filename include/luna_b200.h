@@ -133,7 +133,9 @@ typedef struct {
     int dist_min_no;                           /* batches: instances with at least this many
                                                   oversampled samples run on a cluster of CTAs
                                                   each (in the batch's precision); 0: 4096 in
-                                                  full precision, 16384 in mixed             */
+                                                  full precision (envelope grids; 512 sample
+                                                  pairs a CTA make it 8192 on real ones),
+                                                  16384 in mixed                             */
 } luna_solve_opts;
 
 /* Per-step statistics (Stats.default, Stats.jl:495-532, for a mode-averaged field-resolved

@@ -134,7 +134,8 @@ def schedule(params, probs, table, nsm):
         if row.get("cluster"):
             cluster[i] = w[i] * row["cluster"]
         elif not row.get("single") and p.grid.No >= 16384:
-            cluster[i] = single[i] / 2.0  # untimed long grid: assume the typical cluster gain
+            # an untimed grid that takes clusters in either precision: assume the typical gain
+            cluster[i] = single[i] / 2.0
         if row.get("cluster16"):
             cluster16[i] = w[i] * row["cluster16"]
     mean_load = single.sum() / max(1, nsm)

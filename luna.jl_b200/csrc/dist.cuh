@@ -112,9 +112,10 @@ __device__ __forceinline__ cpx<double> tws_half(int a) {
 
 // Cluster barrier, then buf[n1] *= exp(-+2 pi i f n1 / 2^lg) for this CTA's sub-transform f: the
 // twiddles of the FP64 radix steps on the receiving side, one a thread. The CTAs that form the
-// steps have 32 threads at work (Mb = 512, R = 16), and their R - 1 lookups between remote stores took
-// 8 k of the 21 k cycles of a 16384-point transform. (A DFT over R lanes of a warp, on every thread,
-// loses that again to remote accesses of R different CTAs in one instruction.)
+// steps have 32 threads at work (Mb = 512, R = 16), and made R - 1 lookups between remote stores: without
+// them a right-hand side of 32768 points with Raman went from 74 to 63.5 us. (A DFT over R lanes of a
+// warp, on every thread, gains little more there, 61.2 us, and loses on shorter grids to remote accesses
+// of R different CTAs in one instruction: No = 4096 24.6 to 26.6 us.)
 __device__ __forceinline__ void dsync_twiddle(const TwTab<double>& tw, cpx<double>* b0, int f0, cpx<double>* b1, int f1,
                                               int Mb, int lg) {
     const int tid = threadIdx.x;

@@ -131,8 +131,7 @@ __device__ __forceinline__ void apply_twiddles(cpx<R>* v, cpx<R> w) {
 // TWS_OFF of the CTA's dynamic shared memory (swizzled like the buffers). A radix-8 pass of span
 // L reads w = exp(-2 pi i k/(8 L)), entry k * 512/L, and w^2, and forms the other powers in one or
 // two products. Filled by every kernel that transforms (tws_fill); a pass then waits for shared
-// memory (~30 cycles) instead of L2 (~600 cycles, the L1 being what the buffers leave of 256 KB),
-// and its twiddles carry one to three roundings instead of three to seven (table product, then
+// memory instead of L2 (the L1 being what the buffers leave of 256 KB), and its twiddles carry one to three roundings instead of three to seven (table product, then
 // powers). The FP32 transforms keep their tables in global memory: their pass radices, and so
 // their rounding, are those of the mixed-precision results.
 #define TWS_OFF 2048
@@ -261,12 +260,11 @@ __device__ __forceinline__ void join_pass(cpx<R>* buf, int M, const TwTab<R>& tw
 // buffer in the CTA's dynamic shared memory. What bounds a pass is latency (two barriers, a
 // twiddle lookup and shared-memory round trips at 8-16 active warps), so it must not also wait
 // for local memory or L2. Inlined into the solvers at their 128-register limit (64 in the FP32
-// column kernel), with every radix in one function, the passes spilled 600-2500 bytes a thread:
-// a 2048-point FP64 transform on 512 threads took 18-22 k cycles inside a right-hand side,
-// against 5.1 k alone as functions that keep a butterfly in registers, address shared memory
-// directly and (FP64) read their twiddles there; 9-12 k inside a right-hand side, where the
-// caller's registers are saved around them. The FP32 passes take the same radices, twiddles and
-// operations as before, so their results do not change.
+// column kernel), with every radix in one function, the passes spilled 600-2500 bytes a thread;
+// as functions they keep a butterfly in registers, address shared memory directly and (FP64) read
+// their twiddles there (with plasma_real_f64 and local_inst a right-hand side of 4096 points on one CTA
+// went from 51 to 31 us). The FP32 passes take the same radices, twiddles and operations as before, so
+// their results do not change.
 template <typename R>
 __device__ __forceinline__ unsigned dsm_off(const cpx<R>* p) {
     return (unsigned)__cvta_generic_to_shared(p) - (unsigned)__cvta_generic_to_shared(dsm);

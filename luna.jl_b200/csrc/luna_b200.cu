@@ -911,8 +911,8 @@ int dist_partition(luna_batch* b, const double* pr) {
     return LUNA_OK;
 }
 
-// Distributed instances of a batch: the long ones (No >= dist_min_no, default 16384) that
-// the cluster solver supports, each on DIST_R CTAs, in the batch's precision (FP32 or FP64
+// Distributed instances of a batch: the long ones (No >= dist_min_no, default 4096 in FP64 and 16384 in
+// mixed precision) that the cluster solver supports (dist_fits: real grids from 8192 points in FP64), each on DIST_R CTAs, in the batch's precision (FP32 or FP64
 // sub-transforms and responses). Sets b->elig and the partition when at least one cluster
 // fits on the device; a batch without eligible instances is left unchanged.
 template <typename Rl>
