@@ -1904,6 +1904,7 @@ struct luna_radial_plan {
     char* gscr = nullptr;            // per-column scratch when a column does not fit in shared memory
     size_t gstride = 0;
     int smem = 0;                    // dynamic shared memory of the column kernels
+    int nsm = sm_count();            // (asked once: a query a launch is a fifth of a small product)
     void* A = nullptr;               // [Nw*Nr] stage input, then column output
     void* B = nullptr;               // [Nw*Nr] QDHT output
     int* d_flags = nullptr;
@@ -1971,16 +1972,17 @@ void launch_pdl(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStr
 
 // Er = A Mi^T or Pk = Pw Mf^T along the radial index of the 2Nw x Nr real view: FP64
 // CUDA-core tiles for the plain path, 3xBF16 tensor-core products for the mixed path. FP64 takes
-// 32 x 32 tiles while all of them run at one time (three an SM), 64 x 64 above, whose fewer
-// shared-memory reads a product then count. Tile of 64 against 32 at 2 Nw x Nr, us: 514 x 64 7.2 / 3.7,
-// 2050 x 128 12.7 / 9.0, 2050 x 192 (390 tiles of 32) 18.2 / 17.7, 4098 x 128 (516) 12.9 / 21.7,
-// 2050 x 256 (520) 23.6 / 41.1, 4098 x 384 87.4 / 111.3.
+// 64 x 64 tiles where they occupy half the SMs (fewer shared-memory reads a product), 32 x 32 below. Whole
+// right-hand sides with Kerr in tiles of 64 and 32 at 2 Nw x Nr (tiles of 64), us: 514 x 64 (9) 29.3, 22.0;
+// 2050 x 128 (66) 68.7, 61.0; 2050 x 160 (99) 73.4, 81.2; 2050 x 192 (99) 79.5, 88.8; 2050 x 200 (132) 95.7,
+// 102.0; 4098 x 320 (325) 248, 267. Padding moves single sizes across the line: 4098 x 64 (65) 50.4, 55.9;
+// 2050 x 144 (99) 77.3, 68.6; the product alone crosses at 390 to 450 tiles of 32 (18.2, 17.7; 19.2, 34.9).
 int rad_qdht(luna_radial_plan* p, const void* X, bool fwd, void* Y, const RadState* st, int* flags, cudaStream_t s) {
     const int rows = 2 * p->Nw;
     if (p->precision == LUNA_PREC_FP64) {
-        const int g32 = (rows + 31) / 32 * ((p->Nr + 31) / 32);
+        const int g64 = (rows + 63) / 64 * ((p->Nr + 63) / 64);
         const double* Mx = fwd ? p->Mf : p->Mi;
-        if (g32 > 3 * sm_count())
+        if (2 * g64 >= p->nsm)
             launch_pdl(rad_gemm_f64<64>, dim3((rows + 63) / 64, (p->Nr + 63) / 64), 256, 0, s, (const double*)X, rows, rows, Mx,
                        (double*)Y, p->Nr, st);
         else
